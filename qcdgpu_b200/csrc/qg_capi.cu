@@ -68,6 +68,7 @@ struct qg_ctx {
     bool slab = false;
     int slab_x0 = 0, slab_n1 = 0;
     unsigned long long *d_bad = nullptr;   // qg_field_check counter
+    RefStage stage;                 // reference-layout table copies (lazy)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_phase[8] = {};
     // learned-proposal Metropolis (qg_net_*, qg_mh_*)
@@ -238,6 +239,7 @@ extern "C" int qg_destroy(qg_ctx *c)
     cudaFree(c->d_wpart); cudaFree(c->d_wout);
     cudaFree(c->d_fpart); cudaFree(c->d_ppart); cudaFree(c->d_pout); cudaFree(c->d_sites);
     cudaFree(c->d_bad);
+    ref_stage_free(c->stage);
     if (c->h_results) cudaFreeHost(c->h_results);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_ring) cudaFreeHost(c->h_ring);
@@ -1558,14 +1560,8 @@ extern "C" int qg_links_upload(qg_ctx *c, const void *host, int layout)
 {
     if (!c || !host) return QG_ERR_ARG;
     if (layout != QG_LAYOUT_REFERENCE) return fail(c, QG_ERR_ARG, "unknown layout");
-    const size_t rsz = c->cfg.precision ? sizeof(double) : sizeof(float);
-    const size_t bytes = (size_t)(c->cfg.group == 3 ? 12 : 4) * c->rowsize * 4 * rsz;
-    void *tmp = nullptr;
-    QG_CK(cudaMallocAsync(&tmp, bytes, c->stream), "upload staging");
-    cudaError_t e = cudaMemcpyAsync(tmp, host, bytes, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = launch_to_native(c->G, tmp, c->links, c->cfg.group, c->cfg.precision, c->rowsize, c->stream);
-    cudaFreeAsync(tmp, c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "links upload");
+    QG_CK(ref_stage_copy(c->G, c->links, c->cfg.group, c->cfg.precision, c->rowsize, const_cast<void *>(host), false,
+                         c->stage, c->stream), "links upload");
     QG_CK(cudaStreamSynchronize(c->stream), "upload sync");
     return QG_OK;
 }
@@ -1574,15 +1570,8 @@ extern "C" int qg_links_download(qg_ctx *c, void *host, int layout)
 {
     if (!c || !host) return QG_ERR_ARG;
     if (layout != QG_LAYOUT_REFERENCE) return fail(c, QG_ERR_ARG, "unknown layout");
-    const size_t rsz = c->cfg.precision ? sizeof(double) : sizeof(float);
-    const size_t bytes = (size_t)(c->cfg.group == 3 ? 12 : 4) * c->rowsize * 4 * rsz;
-    void *tmp = nullptr;
-    QG_CK(cudaMallocAsync(&tmp, bytes, c->stream), "download staging");
-    cudaError_t e = cudaMemsetAsync(tmp, 0, bytes, c->stream);
-    if (e == cudaSuccess) e = launch_to_ref(c->G, c->links, tmp, c->cfg.group, c->cfg.precision, c->rowsize, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(host, tmp, bytes, cudaMemcpyDeviceToHost, c->stream);
-    cudaFreeAsync(tmp, c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "links download");
+    QG_CK(ref_stage_copy(c->G, c->links, c->cfg.group, c->cfg.precision, c->rowsize, host, true, c->stage, c->stream),
+          "links download");
     QG_CK(cudaStreamSynchronize(c->stream), "download sync");
     return QG_OK;
 }

@@ -315,42 +315,99 @@ cudaError_t launch_field_check(const Geom &G, const void *links, int group, int 
 }
 
 // ---------------------------------------------------------- layout convert
-template <typename V>
-__global__ void k_to_native(Geom G, const V *ref, V *nat, int planes, uint32_t rowsize)
+// Sites [s0, s1) of planes plane0 .. plane0 + gridDim.y - 1 between the
+// checkerboarded field and a piece of the reference-layout table
+// (TO_REF: padding sites V .. rowsize-1 written as zeros).  Bound by the
+// bytes: a warp's field access is two runs of one parity and its table
+// access one run, all whole sectors; one plane per thread (not a loop over
+// all planes) keeps enough loads in flight and lets the piece be any part
+// of the table.
+template <typename V, bool TO_REF>
+__global__ void __launch_bounds__(256) k_ref_piece(Geom G, V *nat, V *ref, int plane0, uint32_t s0, uint32_t s1)
 {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= G.V) return;
-    Crd c = lex2crd(G, s);
-    uint32_t e = native_index(G, s, c);
-    for (int k = 0; k < planes; k++) nat[(size_t)k * G.pstride + e] = ref[s + (size_t)k * rowsize];
-}
-template <typename V>
-__global__ void k_to_ref(Geom G, const V *nat, V *ref, int planes, uint32_t rowsize)
-{
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= G.V) return;
-    Crd c = lex2crd(G, s);
-    uint32_t e = native_index(G, s, c);
-    for (int k = 0; k < planes; k++) ref[s + (size_t)k * rowsize] = nat[(size_t)k * G.pstride + e];
+    const uint32_t s = s0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= s1) return;
+    V *r = ref + (size_t)blockIdx.y * (s1 - s0) + (s - s0);
+    if (s >= G.V) {
+        if (TO_REF) *r = V{};
+        return;
+    }
+    V *n = nat + (size_t)(plane0 + blockIdx.y) * G.pstride + native_index(G, s, lex2crd(G, s));
+    if (TO_REF) *r = *n; else *n = *r;
 }
 
-cudaError_t launch_to_native(const Geom &G, const void *ref, void *links, int group, int prec, uint32_t rowsize,
-                             cudaStream_t s)
+template <bool TO_REF>
+static cudaError_t launch_ref_piece(const Geom &G, void *links, void *ref, int prec, int plane0, int planes, uint32_t s0,
+                                    uint32_t s1, cudaStream_t s)
 {
-    unsigned nb = (G.V + 127) / 128;
-    int planes = group == 3 ? 12 : 4;
-    if (prec) k_to_native<double4><<<nb, 128, 0, s>>>(G, (const double4 *)ref, (double4 *)links, planes, rowsize);
-    else k_to_native<float4><<<nb, 128, 0, s>>>(G, (const float4 *)ref, (float4 *)links, planes, rowsize);
+    const dim3 grid((s1 - s0 + 255) / 256, (unsigned)planes);
+    if (prec) k_ref_piece<double4, TO_REF><<<grid, 256, 0, s>>>(G, (double4 *)links, (double4 *)ref, plane0, s0, s1);
+    else k_ref_piece<float4, TO_REF><<<grid, 256, 0, s>>>(G, (float4 *)links, (float4 *)ref, plane0, s0, s1);
     return cudaGetLastError();
 }
-cudaError_t launch_to_ref(const Geom &G, const void *links, void *ref, int group, int prec, uint32_t rowsize,
-                          cudaStream_t s)
+
+// The reference-layout link table to or from host memory through a staging
+// buffer that the owner of the field keeps (at most kRefStageBytes; smaller
+// when the table is, or when that much is not free): whole planes, or
+// pieces of one plane, each converted and copied in stream order.  A buffer
+// of the whole table from the stream-ordered pool was unmapped at every
+// synchronisation and mapped again by the next call (a 32^4 FP32 table of
+// 201 MB in, checked, reunitarised, measured and out: 14.6 ms so, 7.8 ms
+// with the kept buffer; a 98 KB one at 4^4 in a 0.66 ms pass: 0.19 ms); the
+// conversion of a piece (about 10 us) is not worth a second buffer beside
+// its copy (1.2 ms at 64 MiB).
+constexpr size_t kRefStageBytes = (size_t)64 << 20, kRefStageMin = (size_t)1 << 20;
+
+void ref_stage_free(RefStage &st)
 {
-    unsigned nb = (G.V + 127) / 128;
-    int planes = group == 3 ? 12 : 4;
-    if (prec) k_to_ref<double4><<<nb, 128, 0, s>>>(G, (const double4 *)links, (double4 *)ref, planes, rowsize);
-    else k_to_ref<float4><<<nb, 128, 0, s>>>(G, (const float4 *)links, (float4 *)ref, planes, rowsize);
-    return cudaGetLastError();
+    cudaFree(st.p);
+    st = RefStage{};
+}
+
+cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
+                           RefStage &st, cudaStream_t s)
+{
+    const size_t es = prec ? sizeof(double4) : sizeof(float4);
+    const int planes = group == 3 ? 12 : 4;
+    const size_t plane_bytes = (size_t)rowsize * es, total = plane_bytes * planes;
+    const size_t want = total < kRefStageBytes ? total : kRefStageBytes;
+    if (st.bytes < want && !st.reduced) {
+        ref_stage_free(st);
+        size_t n = want;
+        cudaError_t e = cudaMalloc(&st.p, n);
+        while (e == cudaErrorMemoryAllocation && n / 2 >= kRefStageMin) {
+            cudaGetLastError();                          // not left pending for the next launch check
+            n /= 2;
+            st.reduced = true;
+            e = cudaMalloc(&st.p, n);
+        }
+        if (e != cudaSuccess) {
+            st = RefStage{};
+            return e;
+        }
+        st.bytes = n;
+    }
+    const int step = (int)(st.bytes / plane_bytes);      // whole planes at a time; 0: pieces of one plane
+    const uint32_t piece = step ? rowsize : (uint32_t)(st.bytes / es);
+    char *h = static_cast<char *>(host);
+    for (int p = 0; p < planes; p += step ? step : 1) {
+        const int np = step ? (planes - p < step ? planes - p : step) : 1;
+        for (uint32_t s0 = 0; s0 < rowsize;) {
+            const uint32_t s1 = rowsize - s0 > piece ? s0 + piece : rowsize;
+            const size_t bytes = (size_t)np * (s1 - s0) * es;
+            char *hp = h + (size_t)p * plane_bytes + (size_t)s0 * es;
+            cudaError_t e;
+            if (to_host) {
+                if ((e = launch_ref_piece<true>(G, links, st.p, prec, p, np, s0, s1, s)) != cudaSuccess) return e;
+                if ((e = cudaMemcpyAsync(hp, st.p, bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+            } else {
+                if ((e = cudaMemcpyAsync(st.p, hp, bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
+                if ((e = launch_ref_piece<false>(G, links, st.p, prec, p, np, s0, s1, s)) != cudaSuccess) return e;
+            }
+            s0 = s1;
+        }
+    }
+    return cudaSuccess;
 }
 
 // ------------------------------------------------------------ observables

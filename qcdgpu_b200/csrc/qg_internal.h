@@ -38,10 +38,18 @@ enum InitKind { INIT_COLD = 0, INIT_GID = 1, INIT_HOT_REF = 2, INIT_HOT_PHILOX =
 cudaError_t launch_init(const Geom &G, void *links, int group, int prec, int kind, int dir,
                         const float4 *prns, uint32_t rowsize, uint2 key, cudaStream_t s);
 cudaError_t launch_gramschmidt(const Geom &G, void *links, int group, int prec, int fp64, cudaStream_t s);
-cudaError_t launch_to_native(const Geom &G, const void *ref, void *links, int group, int prec, uint32_t rowsize,
-                             cudaStream_t s);
-cudaError_t launch_to_ref(const Geom &G, const void *links, void *ref, int group, int prec, uint32_t rowsize,
-                          cudaStream_t s);
+// the staging buffer of reference-layout table copies, kept by the owner of
+// the field (reduced: the wanted size was not free)
+struct RefStage {
+    void *p = nullptr;
+    size_t bytes = 0;
+    bool reduced = false;
+};
+void ref_stage_free(RefStage &st);
+// the field as the reference-layout table in host memory (to_host), or that
+// table into the field; queued on s
+cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
+                           RefStage &st, cudaStream_t s);
 
 // measurements: per-block partials into scratch, then a fixed-order final
 // reduction into out (device).  Partials sizes returned by *_blocks().
