@@ -75,8 +75,10 @@ struct qg_ctx {
     uint16_t *d_netw = nullptr;     // BF16 weights the kernels read
     float *d_master = nullptr, *d_adam_m = nullptr, *d_adam_v = nullptr;
     float *d_grad = nullptr, *d_gpart = nullptr;    // QG_NET_PARAMS + 4 stats; per-block partials
-    double *d_wpart = nullptr, *d_wout = nullptr;   // all-loops Wilson measurement (lazy)
+    double *d_wpart = nullptr;      // all-loops Wilson measurement, column kernel (lazy)
     int wpart_rmax = 0;
+    double *d_wline = nullptr;      // the same: results, and slots and scratch of the time-line gauge (lazy)
+    size_t wline_bytes = 0;
     double *d_fpart = nullptr, *d_ppart = nullptr, *d_pout = nullptr;   // F_munu / profiles (lazy)
     double *d_sites = nullptr;      // per-site values of the one-pass measurements (lazy)
     unsigned long long *d_mh_acc = nullptr;
@@ -236,7 +238,7 @@ extern "C" int qg_destroy(qg_ctx *c)
     cudaFree(c->d_netw); cudaFree(c->d_master); cudaFree(c->d_adam_m); cudaFree(c->d_adam_v);
     cudaFree(c->d_grad); cudaFree(c->d_gpart); cudaFree(c->d_mh_acc); cudaFree(c->d_mh_jump);
     cudaFree(c->d_net_err); cudaFree(c->d_eps);
-    cudaFree(c->d_wpart); cudaFree(c->d_wout);
+    cudaFree(c->d_wpart); cudaFree(c->d_wline);
     cudaFree(c->d_fpart); cudaFree(c->d_ppart); cudaFree(c->d_pout); cudaFree(c->d_sites);
     cudaFree(c->d_bad);
     ref_stage_free(c->stage);
@@ -1382,17 +1384,63 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
         return fail(c, QG_ERR_ARG, "Wilson loop extents must be in [1, 16] and within the lattice");
     const qg_config &f = c->cfg;
     int tw = !(f.phi == 0.0 && f.omega == 0.0);
+    const int nl = Rmax * Tmax;
+    // The time-line gauge (qg_wilson.cu; FP64 products whatever fp64_products
+    // says) costs a preparation and little per loop, the column kernel two
+    // products per loop and R (R - 1) / 2 for the lines.  At SU(3) 32^4 FP32
+    // the gauge takes 1.27 ms + 0.19 ms per R, the column kernel 0.24 / 0.18
+    // ms (FP64 / FP32 products) for 1 x 1, 1.50 / 0.80 for 1 x 8, 2.11 / 1.27
+    // for 8 x 1 and 12.8 / 5.6 for 8 x 8: they cross near R T = 16 with FP64
+    // products (4 x 4: 1.99 against 2.46 ms) and 32 with FP32 ones (5 x 5:
+    // 2.34 against 2.07, 4 x 7: 2.11 against 2.37).  On up to 8^4 sites both
+    // are latency (4^4, 4 x 4: 53 us either way; 8^4, 5 x 5: 65 against 89 us
+    // whatever the products).  The column kernel also
+    // where a line is larger than the scratch, the scratch is not free, or a
+    // time line is too far from SU(N) to be inverted.  One buffer: results
+    // (257), slots, scratch
+    const bool gauge = nl >= (c->G.V <= 4096 ? 25 : (f.precision || fp64_products) ? 16 : 32);
+    const size_t scratch = gauge ? wilson_lines_scratch(c->G, f.group, Tmax) : 0;
+    const size_t head = (257 + wilson_lines_slots(Rmax, Tmax) + 31) / 32 * 32 * sizeof(double);     // 256-byte aligned
+    const size_t want = scratch ? head + scratch : 257 * sizeof(double);
+    if (want > c->wline_bytes) {
+        cudaFree(c->d_wline);
+        c->d_wline = nullptr;
+        c->wline_bytes = 0;
+        cudaError_t e = cudaMalloc(&c->d_wline, want);
+        size_t got = want;
+        if (e == cudaErrorMemoryAllocation && scratch) {
+            cudaGetLastError();
+            got = 257 * sizeof(double);
+            e = cudaMalloc(&c->d_wline, got);
+        }
+        QG_CK(e, "wilson scratch");
+        c->wline_bytes = got;
+    }
+    double *d_wout = c->d_wline;
+    if (scratch && c->wline_bytes >= want) {
+        QG_CK(launch_wilson_lines(c->G, c->links, f.group, f.precision, Rmax, Tmax, c->d_params, tw,
+                                  c->d_wline + head / sizeof(double), scratch, c->d_wline + 257, d_wout, c->stream),
+              "wilson all");
+        double h[257];
+        QG_CK(cudaMemcpyAsync(h, d_wout, (size_t)(nl + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
+              "wilson copy");
+        QG_CK(cudaStreamSynchronize(c->stream), "wilson sync");
+        if (h[nl] == 0.0) {
+            memcpy(out, h, (size_t)nl * sizeof(double));
+            return QG_OK;
+        }
+    }
     if (c->wpart_rmax < Rmax) {
         cudaFree(c->d_wpart);
         c->d_wpart = nullptr;
+        c->wpart_rmax = 0;
         QG_CK(cudaMalloc(&c->d_wpart, wilson_all_partials(wilson_all_blocks(c->G), Rmax) * sizeof(double)),
               "wilson scratch");
         c->wpart_rmax = Rmax;
     }
-    if (!c->d_wout) QG_CK(cudaMalloc(&c->d_wout, 256 * sizeof(double)), "wilson scratch");
     QG_CK(launch_wilson_all(c->G, c->links, f.group, f.precision, Rmax, Tmax, fp64_products, c->d_params, tw,
-                            c->d_wpart, c->d_wout, c->stream), "wilson all");
-    QG_CK(cudaMemcpyAsync(out, c->d_wout, (size_t)Rmax * Tmax * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
+                            c->d_wpart, d_wout, c->stream), "wilson all");
+    QG_CK(cudaMemcpyAsync(out, d_wout, (size_t)nl * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
           "wilson copy");
     QG_CK(cudaStreamSynchronize(c->stream), "wilson sync");
     return QG_OK;

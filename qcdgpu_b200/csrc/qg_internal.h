@@ -87,6 +87,16 @@ size_t wilson_all_partials(int nbx, int Rmax);
 cudaError_t launch_wilson_all(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
                               int fp64_products, const double *params, int twist, double *partials, double *out,
                               cudaStream_t s);
+// all loops in the time-line gauge (qg_wilson.cu): scratch of
+// wilson_lines_scratch bytes (0: a line does not fit, take
+// launch_wilson_all), slots of wilson_lines_slots doubles; out holds
+// Rmax Tmax sums and then a flag, non-zero when a time line is too far from
+// SU(N) for its inverse to be taken (the sums are then not to be used)
+size_t wilson_lines_scratch(const Geom &G, int group, int Tmax);
+size_t wilson_lines_slots(int Rmax, int Tmax);
+cudaError_t launch_wilson_lines(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
+                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *slots,
+                                double *out, cudaStream_t s);
 cudaError_t launch_add_u64(uint64_t *p, uint64_t v, cudaStream_t s);
 // slab halo exchange: both sides of one (direction, parity) slice in one
 // launch; `unit` = 16-byte words per link-plane element, src / dst offsets

@@ -1,0 +1,82 @@
+"""All planar loops in the time-line gauge against the single-loop kernel
+(which multiplies each loop's links up), where the two could part: loop
+extents at the edges of the kernel's blocks of T, time extents split into
+windows, several chunks of lines, links off SU(N), time lines that have no
+inverse."""
+import numpy as np
+import pytest
+
+import qcdgpu_b200 as Q
+
+pytestmark = pytest.mark.gpu
+
+
+def lattice(group, size, precision, sweeps=2, **kw):
+    L = Q.Lattice(Q.default_config(group=group, size=size, precision=precision, start=Q.START_HOT,
+                                   prng=Q.PRNG_PHILOX, beta=5.8 if group == 3 else 2.4, randseries=11, **kw))
+    L.seed()
+    L.init(Q.START_HOT)
+    L.sweep(sweeps)
+    return L
+
+
+def check(L, Rmax, Tmax, loops, fp64=True):
+    W = L.wilson_all(Rmax, Tmax, fp64_products=fp64)
+    V = float(L.info().sites)
+    for R, T in loops:
+        w = L.wilson_sum(R, T)
+        # FP64 products of up to R + T links with growing time lines: 1e-15 a factor on traces of size N,
+        # as random errors of 3 V terms
+        assert abs(W[R - 1, T - 1] - w) <= 1e-14 * 3 * V * L.cfg.group, (R, T, W[R - 1, T - 1], w)
+    return W
+
+
+@pytest.mark.parametrize("group,size,precision,rt", [
+    (3, (2, 2, 2, 2), 1, (2, 2)),            # the column kernel: the smallest, the last below each limit
+    (3, (8, 8, 8, 8), 1, (4, 6)),
+    (3, (8, 6, 8, 12), 1, (3, 5)),
+    (3, (8, 6, 8, 12), 1, (4, 4)),           # the gauge: T = 4, 5, 8, 9, 16, the edges of the blocks of T
+    (2, (12, 10, 8, 10), 1, (4, 5)),
+    (3, (8, 8, 8, 8), 0, (8, 8)),            # the halo is as long as the lattice
+    (2, (6, 6, 6, 18), 0, (3, 9)),
+    (3, (4, 4, 4, 16), 1, (4, 16)),
+    (2, (10, 10, 10, 66), 1, (10, 3)),       # time extents split into windows, the last one ragged
+    (3, (2, 2, 2, 150), 0, (2, 16)),
+    (3, (24, 24, 24, 22), 0, (6, 3)),        # several chunks of lines, breaking inside a direction
+])
+def test_loops_equal_the_single_loops(group, size, precision, rt):
+    L = lattice(group, size, precision)
+    R, T = rt
+    check(L, R, T, [(1, 1), (R, 1), (1, T), (R, T), (R, max(1, T - 1)), (max(1, R - 1), T)])
+    check(L, 1, 1, [(1, 1)])
+    L.close()
+
+
+def test_repeated_calls_of_other_extents_share_the_scratch():
+    """a larger call between two equal ones leaves the second the first's bits"""
+    L = lattice(3, (6, 6, 8, 10), 0)
+    a, b = L.wilson_all(3, 2), L.wilson_all(5, 5)
+    L.wilson_all(6, 10)
+    assert np.array_equal(L.wilson_all(3, 2), a) and np.array_equal(L.wilson_all(5, 5), b)
+    L.close()
+
+
+@pytest.mark.parametrize("twist", [(0.0, 0.0), (0.4, 0.9)])
+def test_links_off_su3(twist):
+    """rows scaled by up to 3 %: the loops are products of the stored links,
+    whatever their departure from SU(3)"""
+    L = lattice(3, (6, 4, 6, 8), 1, phi=twist[0], omega=twist[1])      # 4 x 8 loops: the gauge
+    t = L.download()
+    L.upload(t * (1 + 0.01 * np.random.default_rng(3).standard_normal(t.size).clip(-3, 3)))
+    check(L, 4, 8, [(1, 1), (4, 8), (2, 5), (3, 1)])
+    L.close()
+
+
+def test_time_lines_without_an_inverse_take_the_general_path():
+    """a field of zeros (a context that was never started) has sums 0"""
+    L = Q.Lattice(Q.default_config(group=3, size=(6, 6, 6, 6), precision=0, prng=Q.PRNG_PHILOX))
+    assert np.all(L.wilson_all(5, 5) == 0.0) and np.all(L.wilson_all(5, 5, fp64_products=False) == 0.0)
+    L.seed()
+    L.init(Q.START_COLD)
+    assert np.all(L.wilson_all(6, 6) == 3 * 3 * 6 ** 4)
+    L.close()
