@@ -68,6 +68,7 @@ k_phase_batch(const EnsDesc *ens, const uint32_t *pre, int n, int parity, const 
     A.t_begin = 0;
     A.t_end = G.half;
     A.t_prn = 0;
+    A.after_phase = 0;
     Field<Real> U;
     U.p = reinterpret_cast<typename V4<Real>::T *>(d.links);
     U.pstride = G.pstride;
@@ -187,6 +188,7 @@ __device__ __forceinline__ void tiles_of_phase(const EnsDesc *ens, const uint32_
         A.t_begin = 0;
         A.t_end = G.half;
         A.t_prn = 0;
+        A.after_phase = 0;
         Field<Real> U;
         U.p = reinterpret_cast<typename V4<Real>::T *>(d.links);
         U.pstride = G.pstride;

@@ -567,6 +567,7 @@ static PhaseArgs phase_args(qg_ctx *c, int parity, int dir, int kind, uint32_t o
     a.t_begin = 0;
     a.t_end = c->G.half;
     a.t_prn = 0;
+    a.after_phase = 0;
     if (c->slab) {
         // interior slices 1..w only; the global lattice's thread indices
         // and parity (global x = local x + x0 - 1)
@@ -797,8 +798,11 @@ static cudaError_t enqueue_sweep(qg_ctx *c, bool reunit, cudaEvent_t *ev = nullp
     cudaError_t e;
     uint32_t hb = 0;
     int k_ph = 0;
-    auto timed_phase = [&](const PhaseArgs &a) {
+    auto timed_phase = [&](PhaseArgs a) {
         cudaError_t r;
+        // the launch before this one on the stream is a phase of this graph
+        // (not a batch of the RANLUX stream, not an event)
+        a.after_phase = k_ph > 0 && !ev && a.prn_mode != QG_PRNG_RANLUX;
         if (ev && (r = cudaEventRecordWithFlags(ev[2 * k_ph], c->stream, cudaEventRecordExternal)) != cudaSuccess)
             return r;
         if ((r = launch_phase(c, a)) != cudaSuccess) return r;
@@ -857,6 +861,7 @@ static cudaError_t enqueue_sweep_lookahead(qg_ctx *c, bool reunit, int v)
         for (int mu = 0; mu < 4; mu++, k++) {
             PhaseArgs a = phase_args(c, par_order[pi], mu, QG_UPDATE_HEATBATH, 0);
             a.prns = rl_in(c, v, k);
+            a.after_phase = k > 0;
             if ((e = launch_phase(c, a)) != cudaSuccess) return e;
             if ((e = cudaEventRecord(c->ev_phase[k], c->stream)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(c->side, c->ev_phase[k], 0)) != cudaSuccess) return e;
@@ -868,6 +873,7 @@ static cudaError_t enqueue_sweep_lookahead(qg_ctx *c, bool reunit, int v)
         for (int pi = 0; pi < 2; pi++)
             for (int mu = 0; mu < 4; mu++) {
                 PhaseArgs a = phase_args(c, par_order[pi], mu, QG_UPDATE_OVERRELAX, 0);
+                a.after_phase = 1;
                 if ((e = launch_phase(c, a)) != cudaSuccess) return e;
             }
     if (reunit) {

@@ -196,6 +196,7 @@ struct PrnBuffer {
     __device__ __forceinline__ R4<Real> try_quad() { return next(); }
     __device__ __forceinline__ R4<Real> dir_quad() { return next(); }
     __device__ __forceinline__ void skip() { idx += step; }
+    __device__ __forceinline__ void seek(int n) { idx += (uint32_t)n * step; }     // from the first quad
 };
 
 // in-register counter stream: quad k of thread t in phase p is
@@ -214,6 +215,7 @@ struct PrnPhilox {
     __device__ __forceinline__ R4<Real> try_quad() { return next(); }
     __device__ __forceinline__ R4<Real> dir_quad() { return next(); }
     __device__ __forceinline__ void skip() { k++; }
+    __device__ __forceinline__ void seek(int n) { k = (uint32_t)n; }
 };
 
 // INTS=2 deterministic "random" numbers from the site index

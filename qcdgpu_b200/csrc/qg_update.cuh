@@ -239,6 +239,9 @@ __device__ __forceinline__ M3<float> staple3_staged(const Field<float> &U, const
     return mr_unpack(st);
 }
 
+__device__ __forceinline__ void grid_dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // PRN source of thread t (PMODE 0 = RANLUX buffer, 1 = Philox, 2 = gid)
 template <typename Real, int PMODE> struct PrnOf;
 template <typename Real> struct PrnOf<Real, 0> {
@@ -263,6 +266,25 @@ template <typename Real> struct PrnOf<Real, 2> {
         T p; p.g = (double)(float)site; p.V = (double)G.V; p.nhit = A.nhit; return p;
     }
 };
+
+// the SU(2) group's update of link m0 with staple st: a Kennedy-Pendleton
+// draw (m0 stays when no try is accepted) or the reflection
+template <typename Real, bool OR, class Prn>
+__device__ __forceinline__ R4<Real> su2_update(const S2<Real> &st, const R4<Real> &m0, Real beta, Prn &prn, int nhit)
+{
+    if (!OR) {
+        S2<Real> a = st;
+        if (kp_step<Real, false>(a, beta, prn, nhit)) return { a.u1.re, a.u2.re, a.u1.im, a.u2.im };
+        return m0;
+    }
+    Real Mx = st.u1.re + st.v2.re, My = st.u1.im - st.v2.im;
+    Real Mz = st.u2.re - st.v1.re, Mw = st.u2.im + st.v1.im;
+    Real n2 = Mx * Mx;
+    n2 = FMA(My, My, n2); n2 = FMA(Mz, Mz, n2); n2 = FMA(Mw, Mw, n2);
+    Real id = (Real)1 / RC<Real>::sq(n2);
+    R4<Real> aH = { Mx * id, -Mz * id, -My * id, -Mw * id };
+    return times2(times2(aH, herm2(m0)), aH);
+}
 
 // MINB: minimum resident blocks of 128 threads per SM asked of the
 // compiler (0 = its own register choice); the launch shapes the tuner picks
@@ -314,28 +336,16 @@ __device__ __forceinline__ void phase_site(const Field<Real> &U, const Geom &G, 
             m0 = times2(om, m0);
         }
         S2<Real> st = staple2<mu>(U, G, t, nb, p, tw);
-        if (!OR) {
-            S2<Real> a = st;
-            if (kp_step<Real, false>(a, beta, prn, A.nhit))
-                U.st2(mu, e0, R4<Real>{ a.u1.re, a.u2.re, a.u1.im, a.u2.im });
-            else
-                U.st2(mu, e0, m0);
-        } else {
-            Real Mx = st.u1.re + st.v2.re, My = st.u1.im - st.v2.im;
-            Real Mz = st.u2.re - st.v1.re, Mw = st.u2.im + st.v1.im;
-            Real n2 = Mx * Mx;
-            n2 = FMA(My, My, n2); n2 = FMA(Mz, Mz, n2); n2 = FMA(Mw, Mw, n2);
-            Real id = (Real)1 / RC<Real>::sq(n2);
-            R4<Real> aH = { Mx * id, -Mz * id, -My * id, -Mw * id };
-            U.st2(mu, e0, times2(times2(aH, herm2(m0)), aH));
-        }
+        U.st2(mu, e0, su2_update<Real, OR>(st, m0, beta, prn, A.nhit));
     }
 }
 
 template <int NC, typename Real, int PMODE, bool OR, int mu, int MINB, bool STAGED, bool TW>
 __global__ void __launch_bounds__(kPhaseBlock, MINB) k_phase(Field<Real> U, Geom G, PhaseArgs A)
 {
+    grid_dependents_may_start();
     const uint32_t t = A.t_begin + blockIdx.x * blockDim.x + threadIdx.x;
+    grid_dependency_wait();
     if (t >= A.t_end) return;
     if constexpr (STAGED) {
         __shared__ __align__(16) StageBuf sb;
@@ -394,6 +404,299 @@ __global__ void __launch_bounds__(kPhaseBlock, 1) k_phase_or_pair(Field<float> U
     if (two) U.st3(mu, own1, r1);
 }
 
+// -------------------------------------------------- small lattices
+// A phase of few links is bound by one link's chain of latencies (loads, six
+// staple terms, three subgroup draws) and the launch, not by throughput.  SP = 6
+// or 3 warps share 32 links here: each computes one staple term (warp w: plane
+// w / 2, forward or backward) and its share of the sums, and the first one
+// updates the links; in a heatbath the six also evaluate the functions of
+// the first kSplitQuads random quads (logarithms, sines) ahead, so that the
+// updating warp finds them in shared memory (it computes them itself for
+// the rare later quads).  Operations and their order per value are those of
+// phase_site.  In a sweep's graph the launches are programmatic dependents:
+// a phase's indices and random numbers are computed under the end of the
+// phase before it.
+constexpr int kSplitQuads = 6;
+
+// the functions of one quad that a Kennedy-Pendleton step uses, as a try
+// (num = log(1-x) + cos^2(2 pi y) log(1-z), w2 = w^2) and as a direction
+template <typename Real> struct QuadTry { double num; Real w2; };
+template <typename Real> struct QuadDir { Real costh, sinth, sinphi, cosphi; };
+template <typename Real>
+__device__ __forceinline__ QuadTry<Real> quad_try(const R4<Real> &rnd)
+{
+    QuadTry<Real> q;
+    Real cosrnd = RC<Real>::cs(RC<Real>::PI2 * rnd.y);
+    double lx = qg_log(1.0 - (double)rnd.x), lz = qg_log(1.0 - (double)rnd.z);
+    q.num = FMA((double)(cosrnd * cosrnd), lz, lx);
+    q.w2 = rnd.w * rnd.w;
+    return q;
+}
+template <typename Real>
+__device__ __forceinline__ QuadDir<Real> quad_dir(const R4<Real> &rnd)
+{
+    QuadDir<Real> q;
+    q.costh = (Real)FMA(2.0, (double)rnd.x, -1.0);
+    q.sinth = (Real)sqrt(1.0 - (double)(q.costh * q.costh));
+    Real phi = RC<Real>::PI2 * rnd.y;
+    q.sinphi = RC<Real>::sn(phi);
+    q.cosphi = RC<Real>::cs(phi);
+    return q;
+}
+template <typename Real> struct QuadTable {
+    QuadTry<Real> t[kSplitQuads][32];
+    QuadDir<Real> d[kSplitQuads][32];
+};
+// quad k of the link's stream: a table entry, or computed from the source
+template <typename Real, class Src> struct PrnTable {
+    static constexpr bool GID = false;
+    Src src;
+    const QuadTable<Real> *tab;
+    int k, lane;
+    __device__ __forceinline__ R4<Real> quad(int n) { Src s = src; s.seek(n); return s.next(); }
+    __device__ __forceinline__ QuadTry<Real> try_vals()
+    {
+        const int n = k++;
+        return n < kSplitQuads ? tab->t[n][lane] : quad_try(quad(n));
+    }
+    __device__ __forceinline__ QuadDir<Real> dir_vals()
+    {
+        const int n = k++;
+        return n < kSplitQuads ? tab->d[n][lane] : quad_dir(quad(n));
+    }
+    __device__ __forceinline__ void skip() { k++; }
+};
+
+// kp_step with the quads' functions at hand
+template <typename Real, bool SU3PATH, class Src>
+__device__ __forceinline__ bool kp_step(S2<Real> &a, Real beta, PrnTable<Real, Src> &prn, int nhit)
+{
+    R4<Real> aH;
+    aH.x =  (a.u1.re + a.v2.re);
+    aH.z = -(a.u1.im - a.v2.im);
+    aH.y = -(a.u2.re - a.v1.re);
+    aH.w = -(a.u2.im + a.v1.im);
+    Real n2 = aH.x * aH.x;
+    if (SU3PATH) {
+        n2 = FMA(aH.y, aH.y, n2); n2 = FMA(aH.z, aH.z, n2); n2 = FMA(aH.w, aH.w, n2);
+    } else {
+        n2 = FMA(aH.z, aH.z, n2); n2 = FMA(aH.y, aH.y, n2); n2 = FMA(aH.w, aH.w, n2);
+    }
+    const Real det = RC<Real>::sq(n2);
+    const Real id = (Real)1 / det;
+    aH.x *= id; aH.z *= id; aH.y *= id; aH.w *= id;
+    const Real bdet = beta * det;
+    Real delta = 0;
+    bool flag = false;
+    for (int i = 0; i < nhit && !flag; i++) {
+        const QuadTry<Real> q = prn.try_vals();
+        delta = (Real)(-q.num / (double)bdet);
+        if ((double)q.w2 <= FMA(-0.5, (double)delta, 1.0)) flag = true;
+    }
+    if (flag) {
+        const QuadDir<Real> q = prn.dir_vals();
+        Real cosal = (Real)(1.0 - (double)delta);
+        Real sinal = (Real)sqrt(1.0 - (double)(cosal * cosal));
+        R4<Real> c;
+        c.x = cosal;
+        c.z = sinal * q.costh;
+        c.y = sinal * q.sinth * q.sinphi;
+        c.w = sinal * q.sinth * q.cosphi;
+        a = rec2(times2(c, aH));
+        return true;
+    }
+    if (SU3PATH) {
+        a.u1 = { (Real)1, (Real)0 }; a.u2 = { (Real)0, (Real)0 };
+        a.v1 = { (Real)0, (Real)0 }; a.v2 = { (Real)1, (Real)0 };
+        prn.skip();
+    }
+    return false;
+}
+
+template <int NC, typename Real, int PMODE, bool OR, int mu, int SP>
+__global__ void __launch_bounds__(32 * SP) k_phase_split(Field<Real> U, Geom G, PhaseArgs A)
+{
+    constexpr int NT = NC == 3 ? 18 : 4;                // numbers of a term (SU(2): the quaternion)
+    __shared__ Real term[6][NT][32];
+    __shared__ QuadTable<Real> tab;                     // heatbath only
+    grid_dependents_may_start();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t t = A.t_begin + blockIdx.x * 32 + lane;
+    const bool on = t < A.t_end;
+    const int p = A.parity;
+    Crd c = lex2crd(G, 2 * (on ? t : A.t_begin));
+    if (parity_of(c) != p) c.y += 1;
+    const uint32_t site = 2 * t + (uint32_t)(c.y & 1);
+    const Nbr n = neighbours(G, c);
+    const uint32_t own = (uint32_t)p * G.cb + t, opp = (uint32_t)(p ^ 1) * G.cb + t;
+    using PS = PrnOf<Real, PMODE>;
+    typename PS::T src;
+    auto fill = [&]() {
+        for (int k = w; k < kSplitQuads; k += SP) {
+            auto s = src;
+            s.seek(k);
+            const R4<Real> q = s.next();
+            tab.t[k][lane] = quad_try(q);
+            tab.d[k][lane] = quad_dir(q);
+        }
+    };
+    if constexpr (!OR) {
+        src = PS::make(A, t, site, PMODE == 1 ? *A.phase_base + A.phase_offset : 0, G);
+        if (PMODE == 1) fill();                         // no memory of earlier phases is read
+    }
+    grid_dependency_wait();
+    const Real beta = (Real)A.params[0];
+    G3<Real> m0;
+    R4<Real> q0;
+    if (on) {
+        if (w == 0) {
+            if constexpr (NC == 3) m0 = U.ld3(mu, own);
+            else q0 = U.ld2(mu, own);
+        }
+#pragma unroll
+        for (int j = 0; j < 6 / SP; j++) {
+            // forward U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+, backward U_nu(x-nu+mu)^+ U_mu(x-nu)^+ U_nu(x-nu)
+            const int k = w * (6 / SP) + j, nu = nu_of(mu, k >> 1);
+            const bool bwd = k & 1;
+            const int32_t d = bwd ? pick4(n.dm, nu) : pick4(n.dp, nu);
+            const uint32_t ea = bwd ? own + d + n.dp[mu] : opp + n.dp[mu], eb = opp + d, ec = bwd ? opp + d : own;
+            if constexpr (NC == 3) {
+                const G3<Real> ga = U.ld3(nu, ea), gb = U.ld3(mu, eb), gc = U.ld3(nu, ec);
+                M3<Real> T;
+                if constexpr (sizeof(Real) == 4)
+                    T = mr_unpack(bwd ? staple_bwd3_rows(ga, gb, gc) : staple_fwd3_rows(ga, gb, gc));
+                else
+                    T = bwd ? staple_bwd3(ga, gb, gc) : staple_fwd3(ga, gb, gc);
+#pragma unroll
+                for (int i = 0; i < 9; i++) {
+                    term[k][2 * i][lane] = T.m[i / 3][i % 3].re;
+                    term[k][2 * i + 1][lane] = T.m[i / 3][i % 3].im;
+                }
+            } else {
+                const R4<Real> ga = U.ld2(nu, ea), gb = U.ld2(mu, eb), gc = U.ld2(nu, ec);
+                const R4<Real> T =
+                    bwd ? times2(times2(herm2(ga), herm2(gb)), gc) : times2(times2(ga, herm2(gb)), herm2(gc));
+                term[k][0][lane] = T.x;
+                term[k][1][lane] = T.y;
+                term[k][2][lane] = T.z;
+                term[k][3][lane] = T.w;
+            }
+        }
+        if constexpr (!OR && PMODE == 0) fill();
+    }
+    __syncthreads();
+    if (on) {                                           // st = f0 + b0; st = b_i + (st + f_i)
+        for (int k = w; k < NT; k += SP) {
+            Real st = term[0][k][lane] + term[1][k][lane];
+            st = term[3][k][lane] + (st + term[2][k][lane]);
+            st = term[5][k][lane] + (st + term[4][k][lane]);
+            term[0][k][lane] = st;
+        }
+    }
+    __syncthreads();
+    if (w != 0 || !on) return;
+    PrnTable<Real, typename PS::T> prn;
+    if constexpr (!OR) {
+        prn.src = src;
+        prn.tab = &tab;
+        prn.k = 0;
+        prn.lane = lane;
+    }
+    if constexpr (NC == 3) {
+        M3<Real> st;
+#pragma unroll
+        for (int i = 0; i < 9; i++) st.m[i / 3][i % 3] = { term[0][2 * i][lane], term[0][2 * i + 1][lane] };
+        G3<Real> r;
+        if constexpr (OR && sizeof(Real) == 4) r = cm3_or_rows(st, m0, A.nhitpar);
+        else r = cm3<Real, OR>(st, m0, beta, prn, A.nhit, A.nhitpar);
+        U.st3(mu, own, r);
+    } else {
+        const S2<Real> st = rec2(R4<Real>{ term[0][0][lane], term[0][1][lane], term[0][2][lane], term[0][3][lane] });
+        U.st2(mu, own, su2_update<Real, OR>(st, q0, beta, prn, A.nhit));
+    }
+}
+
+// a phase kernel; early: as the programmatic dependent of the phase before it
+// in the graph (the kernels wait for that grid before they read links)
+template <typename Real>
+cudaError_t launch_after(void (*kern)(Field<Real>, Geom, PhaseArgs), unsigned nb, unsigned bs, bool early,
+                         const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStream_t s)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(bs);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, U, G, a);
+}
+
+// Launches k_phase_split with SP warps for 32 links; false where that is not
+// the faster form.  A block's registers stay taken while its first warp alone
+// updates the links, so the split pays while all blocks are resident with
+// room to spare: for SP = 6 up to 3/4 (SU(2): 3/5) of the resident blocks, for
+// SP = 3 up to 3/4 (with RANLUX batches, whose generator wants the SMs too,
+// 1/2).  Measured in the sweep graph, us a phase, heatbath / overrelaxation:
+//   SU(3) FP32  8^4   9.7 / 5.1 -> 6.6 / 2.7    16^3 x 8  10.3 / 5.1 -> 8.4 / 4.4
+//   SU(3) FP64  8^4  11.5 / 6.2 -> 7.0 / 3.6    16^3 x 8  12.1 / 6.5 -> 9.8 / 6.6
+//   SU(2) FP32  8^4   4.9 / 2.7 -> 2.6 / 1.5    16^4       5.5 / 3.1 -> 4.5 / 2.9
+//   SU(2) FP64  8^4   5.9 / 3.5 -> 2.7 / 1.7    16^3 x 8   6.2 / 3.6 -> 4.1 / 2.9
+// and beyond them, unsplit against SP = 3: SU(3) FP32 16^4 11.1 / 5.5 against
+// 13.1 / 6.2, FP64 14.3 / 8.4 against 16.9 / 11.2.  The early launch hides
+// the Philox heatbath's random numbers (SU(2) 8^4: 4.1 -> 2.6 us); without
+// them it only pays up to half a block per SM (the next phase's blocks
+// crowd where the first slots come free: SU(3) FP32 12^3 x 8
+// overrelaxation 3.2 us without, 4.2 with it, 4^4 2.65 / 2.31).
+template <int NC, typename Real, int PM, bool OR, int MU, int SP>
+bool try_split(const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStream_t s, cudaError_t &e)
+{
+    static const int per_sm = [] {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_phase_split<NC, Real, PM, OR, MU, SP>, 32 * SP, 0) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        return n;
+    }();
+    const unsigned nb = (a.t_end - a.t_begin + 31) / 32, resident = 148u * per_sm;
+    const unsigned limit = SP == 6 ? (NC == 3 ? resident * 3 / 4 : resident * 3 / 5)
+                                   : (!OR && PM == 0 ? resident / 2 : resident * 3 / 4);
+    if (nb > limit) return false;
+    const bool early = a.after_phase && ((!OR && PM == 1) || nb <= 74);
+    e = launch_after(k_phase_split<NC, Real, PM, OR, MU, SP>, nb, 32 * SP, early, U, G, a, s);
+    return true;
+}
+
+template <typename Real>
+bool launch_phase_split(const Field<Real> &U, const Geom &G, int group, const PhaseArgs &a, cudaStream_t s,
+                        cudaError_t &e)
+{
+#define QG_SPLIT1(NC, PM, OR, MU)                                                                       \
+    return try_split<NC, Real, PM, OR, MU, 6>(U, G, a, s, e) || try_split<NC, Real, PM, OR, MU, 3>(U, G, a, s, e)
+#define QG_SPLIT(NC, PM, OR)                            \
+    switch (a.dir) {                                    \
+    case 0: QG_SPLIT1(NC, PM, OR, 0);                   \
+    case 1: QG_SPLIT1(NC, PM, OR, 1);                   \
+    case 2: QG_SPLIT1(NC, PM, OR, 2);                   \
+    default: QG_SPLIT1(NC, PM, OR, 3);                  \
+    }
+    if (group == 3) {
+        if (a.prn_mode == -1) { QG_SPLIT(3, 0, true) }
+        else if (a.prn_mode == 0) { QG_SPLIT(3, 0, false) }
+        else { QG_SPLIT(3, 1, false) }
+    } else {
+        if (a.prn_mode == -1) { QG_SPLIT(2, 0, true) }
+        else if (a.prn_mode == 0) { QG_SPLIT(2, 0, false) }
+        else { QG_SPLIT(2, 1, false) }
+    }
+#undef QG_SPLIT
+#undef QG_SPLIT1
+}
+
 template <typename Real>
 cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArgs &a, cudaStream_t s)
 {
@@ -420,13 +723,21 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
             return cudaGetLastError();
         }
     }
+    // many blocks: the next phase's first blocks start in this one's last wave
+    // (32^4: SU(3) FP32 overrelaxation 52.2 -> 50.1 us in shape 1, 52.6 ->
+    // 51.8 in shape 3, SU(2) FP32 11.1 -> 10.6; 24^4 2-4 %); with fewer they
+    // crowd on the SMs whose blocks end first (16^4 5.5 -> 9.6 us)
+    const bool early = a.after_phase && nb >= 1024;
+    // shape 0 of few links: six or three warps for 32 links (k_phase_split)
+    cudaError_t e;
+    if (a.variant == 0 && !a.twist && pm != 2 && launch_phase_split<Real>(U, G, group, a, s, e)) return e;
     // twisted boundaries: shape 0's form with the twist tests compiled in
     // (any shape computes the same sequence); the others are compiled
     // without them
-#define QG_LAUNCH2(NC, PM, OR, MU, MB, ST) k_phase<NC, Real, PM, OR, MU, MB, ST, false><<<nb, bs, 0, s>>>(U, G, a)
+#define QG_LAUNCH2(NC, PM, OR, MU, MB, ST) return launch_after(k_phase<NC, Real, PM, OR, MU, MB, ST, false>, nb, bs, early, U, G, a, s)
 #define QG_LAUNCH1(NC, PM, OR, MU)                                                  \
     do {                                                                            \
-        if (a.twist) k_phase<NC, Real, PM, OR, MU, 0, false, true><<<nb, bs, 0, s>>>(U, G, a); \
+        if (a.twist) return launch_after(k_phase<NC, Real, PM, OR, MU, 0, false, true>, nb, bs, early, U, G, a, s); \
         else if (a.variant == 1) QG_LAUNCH2(NC, PM, OR, MU, 5, false);              \
         else if (a.variant == 2) QG_LAUNCH2(NC, PM, OR, MU, 6, false);              \
         else if (a.variant == 3) QG_LAUNCH2(NC, PM, OR, MU, 0, NC == 3 && kStage);  \
@@ -456,7 +767,6 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
 #undef QG_LAUNCH
 #undef QG_LAUNCH1
 #undef QG_LAUNCH2
-    return cudaGetLastError();
 }
 
 }  // namespace qg

@@ -1,0 +1,60 @@
+"""The small-lattice phase kernel (a link's staple terms over six or three
+warps, shape 0) against the one-thread-per-link kernels (shape 1), link by
+link: blocks that are not full, the sizes on both sides of each limit, long
+reject chains (random quads beyond the precomputed ones), several hits, the
+RANLUX stream, and the graph's early launches against single phases."""
+import numpy as np
+import pytest
+
+import qcdgpu_b200 as Q
+
+pytestmark = pytest.mark.gpu
+
+
+def chain(shape, sweeps, **kw):
+    L = Q.Lattice(Q.default_config(start=Q.START_HOT, randseries=7, reunit_every=2, **kw))
+    L.seed()
+    L.init(Q.START_HOT)
+    L.set_shapes(shape, shape)
+    L.sweep(sweeps)
+    out = L.download()
+    L.close()
+    return out
+
+
+@pytest.mark.parametrize("group", [3, 2])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("size", [(2, 2, 2, 2), (4, 2, 6, 2), (6, 6, 6, 6), (10, 10, 10, 8), (12, 12, 12, 8),
+                                  (16, 16, 16, 8), (16, 16, 16, 14), (20, 20, 20, 14)])
+def test_split_phases_give_the_same_chain(group, precision, size):
+    kw = dict(group=group, precision=precision, size=size, beta=5.9 if group == 3 else 2.3, n_or=2, prng=Q.PRNG_PHILOX)
+    assert np.array_equal(chain(0, 3, **kw), chain(1, 3, **kw))
+
+
+@pytest.mark.parametrize("group,precision", [(3, 0), (3, 1), (2, 0), (2, 1)])
+@pytest.mark.parametrize("prng", [Q.PRNG_PHILOX, Q.PRNG_RANLUX])
+def test_split_phases_rejects_and_hits(group, precision, prng):
+    """strong coupling (most first tries rejected, so the quads run past the
+    table and some draws keep the link) and two hits per subgroup"""
+    kw = dict(group=group, precision=precision, size=(6, 4, 6, 8), beta=0.3, nhit=3, nhitpar=2, n_or=1, prng=prng,
+              prng_instances=512)
+    assert np.array_equal(chain(0, 2, **kw), chain(1, 2, **kw))
+
+
+@pytest.mark.parametrize("prng", [Q.PRNG_PHILOX, Q.PRNG_RANLUX])
+def test_graph_sweeps_equal_single_phases(prng):
+    """the graph launches phases early (their random numbers under the phase
+    before); phase by phase there is nothing to overlap"""
+    kw = dict(group=3, precision=0, size=(8, 8, 8, 8), beta=5.9, prng=prng, prng_instances=2048)
+    L = Q.Lattice(Q.default_config(start=Q.START_HOT, randseries=7, reunit_every=2, **kw))
+    L.seed()
+    L.init(Q.START_HOT)
+    for _ in range(2):
+        for p in (1, 0):
+            for d in range(4):
+                if prng == Q.PRNG_RANLUX:
+                    L.produce()
+                L.phase(p, d)
+    L.reunitarize()
+    assert np.array_equal(L.download(), chain(0, 2, **kw))
+    L.close()
