@@ -27,13 +27,14 @@ struct qg_ctx {
     double *partials = nullptr;
     size_t partials_n = 0;
     double *d_results = nullptr;
-    double *h_results = nullptr;    // pinned
+    double *h_results = nullptr;    // pinned; the observables' kernels write here
+    unsigned *d_ticket = nullptr;   // their block counter (in d_results)
     uint64_t *d_phase = nullptr;
     double *d_params = nullptr;     // {BETA/N, PHI, OMEGA, 0}: lattice_parameters
     double *h_params = nullptr;     // pinned staging, kParamSlots x 4 doubles
     cudaEvent_t param_ev[8] = {};   // slot's upload done
     uint32_t param_next = 0;
-    // asynchronous measurements: pinned result slots, their copy events and tickets
+    // asynchronous measurements: pinned result slots, their events and tickets
     double *h_ring = nullptr;       // QG_MEASURE_SLOTS x 8 doubles
     cudaEvent_t ring_ev[QG_MEASURE_SLOTS] = {};
     uint64_t ring_ticket[QG_MEASURE_SLOTS] = {};
@@ -313,6 +314,8 @@ extern "C" int qg_create(const qg_config *cfg, qg_ctx **out)
     }
     if ((e = cudaMalloc(&c->partials, c->partials_n * sizeof(double))) != cudaSuccess) return bad("cudaMalloc(partials)");
     if ((e = cudaMalloc(&c->d_results, 64 * sizeof(double))) != cudaSuccess) return bad("cudaMalloc(results)");
+    c->d_ticket = reinterpret_cast<unsigned *>(c->d_results + 63);
+    if ((e = cudaMemsetAsync(c->d_ticket, 0, sizeof(double), c->stream)) != cudaSuccess) return bad("cudaMemset(ticket)");
     if ((e = cudaMallocHost(&c->h_results, 64 * sizeof(double))) != cudaSuccess) return bad("cudaMallocHost");
     if ((e = cudaMalloc(&c->d_phase, sizeof(uint64_t))) != cudaSuccess) return bad("cudaMalloc(phase)");
     if ((e = cudaMemsetAsync(c->d_phase, 0, sizeof(uint64_t), c->stream)) != cudaSuccess) return bad("cudaMemset(phase)");
@@ -674,15 +677,15 @@ extern "C" int qg_profile_kernels(qg_ctx *c, int reps, double *mean_ms, double *
                 e = launch_gramschmidt(c->G, c->links, f.group, f.precision, f.reunit_fp64, c->stream);
                 break;
             case QG_KERNEL_PLAQUETTE:
-                e = launch_plaquette(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_results,
-                                     c->stream);
+                e = launch_plaquette(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_ticket,
+                                     c->d_results, c->stream);
                 break;
             case QG_KERNEL_POLYAKOV:
-                e = launch_polyakov(c->G, c->links, f.group, f.precision, c->partials, c->d_results, c->stream);
+                e = launch_polyakov(c->G, c->links, f.group, f.precision, c->partials, c->d_ticket, c->d_results, c->stream);
                 break;
             default:
                 e = launch_wilson(c->G, c->links, f.group, f.precision, f.wilson_r, f.wilson_t, c->d_params, tw,
-                                  c->partials, c->d_results, c->stream);
+                                  c->partials, c->d_ticket, c->d_results, c->stream);
                 break;
             }
             if (r >= 0) cudaEventRecord(ev[2 * r + 1], c->stream);
@@ -1361,10 +1364,9 @@ extern "C" int qg_net_train(qg_ctx *c, int steps, double lr, double *stats)
     return net_err_check(c);
 }
 
+// the values that a measurement's kernel wrote to h_results
 static int measure_to_host(qg_ctx *c, int ncomp, double *out)
 {
-    QG_CK(cudaMemcpyAsync(c->h_results, c->d_results, ncomp * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
-          "result copy");
     QG_CK(cudaStreamSynchronize(c->stream), "measure sync");
     for (int i = 0; i < ncomp; i++) out[i] = c->h_results[i];
     return QG_OK;
@@ -1376,8 +1378,8 @@ extern "C" int qg_measure_wilson(qg_ctx *c, int R, int T, double *out)
     if (R < 1 || T < 1 || R > c->G.n[0] || T > c->G.n[3]) return fail(c, QG_ERR_ARG, "Wilson loop extent out of range");
     const qg_config &f = c->cfg;
     int tw = !(f.phi == 0.0 && f.omega == 0.0);
-    QG_CK(launch_wilson(c->G, c->links, f.group, f.precision, R, T, c->d_params, tw, c->partials, c->d_results,
-                        c->stream), "wilson");
+    QG_CK(launch_wilson(c->G, c->links, f.group, f.precision, R, T, c->d_params, tw, c->partials, c->d_ticket,
+                        c->h_results, c->stream), "wilson");
     return measure_to_host(c, 1, out);
 }
 
@@ -1463,12 +1465,9 @@ extern "C" int qg_measure_fmunu(qg_ctx *c, int field, int index1, int index2, do
         return fail(c, QG_ERR_ARG, "generator index out of range (1..8 for SU(3), 1..3 for SU(2))");
     int tw = !(f.phi == 0.0 && f.omega == 0.0);
     if (!c->d_fpart) QG_CK(cudaMalloc(&c->d_fpart, fmunu_partials(c->G) * sizeof(double)), "fmunu scratch");
-    if (!c->d_pout) QG_CK(cudaMalloc(&c->d_pout, 2 * 4096 * sizeof(double)), "measurement scratch");
     QG_CK(launch_fmunu(c->G, c->links, f.group, f.precision, c->d_params, tw, field, index1, index2, c->d_fpart,
-                       c->d_pout, c->stream), "fmunu");
-    QG_CK(cudaMemcpyAsync(out, c->d_pout, 12 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "fmunu copy");
-    QG_CK(cudaStreamSynchronize(c->stream), "fmunu sync");
-    return QG_OK;
+                       c->d_ticket, c->h_results, c->stream), "fmunu");
+    return measure_to_host(c, 12, out);
 }
 
 static int measure_profile(qg_ctx *c, int kind, int axis, double *out)
@@ -1498,7 +1497,7 @@ static int measure_all(qg_ctx *c, int kind, double *out)
     if (!c->d_pout) QG_CK(cudaMalloc(&c->d_pout, 2 * 4096 * sizeof(double)), "measurement scratch");
     if (!c->d_sites) QG_CK(cudaMalloc(&c->d_sites, sites_buffer_doubles(c->G) * sizeof(double)), "site buffer");
     QG_CK(launch_measure_all(c->G, c->links, f.group, f.precision, c->d_params, tw, kind, c->partials, c->d_ppart,
-                             c->d_sites, c->d_pout, c->stream), "one-pass measurement");
+                             c->d_sites, c->d_ticket, c->d_pout, c->stream), "one-pass measurement");
     QG_CK(cudaMemcpyAsync(out, c->d_pout, (size_t)nout * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
           "measurement copy");
     QG_CK(cudaStreamSynchronize(c->stream), "measurement sync");
@@ -1509,72 +1508,53 @@ extern "C" int qg_measure_polyakov_all(qg_ctx *c, double *out) { return measure_
 extern "C" int qg_measure_action_profile(qg_ctx *c, int axis, double *out) { return measure_profile(c, 0, axis, out); }
 extern "C" int qg_measure_polyakov_profile(qg_ctx *c, int axis, double *out) { return measure_profile(c, 1, axis, out); }
 
-extern "C" int qg_measure(qg_ctx *c, int what, double *out)
-{
-    if (!c || !out) return QG_ERR_ARG;
-    const qg_config &f = c->cfg;
-    int tw = !(f.phi == 0.0 && f.omega == 0.0);
-    switch (what) {
-    case QG_MEAS_PLAQUETTE:
-    case QG_MEAS_ACTION: {
-        QG_CK(launch_plaquette(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_results,
-                               c->stream), "plaquette");
-        double r[4];
-        int rc = measure_to_host(c, 4, r);
-        if (rc) return rc;
-        if (what == QG_MEAS_PLAQUETTE) { out[0] = r[0]; out[1] = r[1]; }
-        else { out[0] = r[2]; out[1] = r[3]; }
-        return QG_OK;
-    }
-    case QG_MEAS_PLAQUETTE_F32:
-        QG_CK(launch_plaquette_f32(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_results,
-                                   c->stream), "plaquette (FP32 products)");
-        return measure_to_host(c, 2, out);
-    case QG_MEAS_POLYAKOV:
-        QG_CK(launch_polyakov(c->G, c->links, f.group, f.precision, c->partials, c->d_results, c->stream), "polyakov");
-        return measure_to_host(c, 4, out);
-    case QG_MEAS_WILSON:
-        return qg_measure_wilson(c, f.wilson_r, f.wilson_t, out);
-    default:
-        return fail(c, QG_ERR_ARG, "unknown measurement");
-    }
-}
-
-// the measurement kernels of `what` into d_results; ncomp values there
-static int measure_launch(qg_ctx *c, int what, int &ncomp, int &first)
+// the measurement kernels of `what`, their values into out (page-locked);
+// ncomp values from out + first are the measurement's
+static int measure_launch(qg_ctx *c, int what, double *out, int &ncomp, int &first)
 {
     const qg_config &f = c->cfg;
     int tw = !(f.phi == 0.0 && f.omega == 0.0);
+    first = 0;
     switch (what) {
     case QG_MEAS_PLAQUETTE:
     case QG_MEAS_ACTION:
-        QG_CK(launch_plaquette(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_results,
+        QG_CK(launch_plaquette(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_ticket, out,
                                c->stream), "plaquette");
         ncomp = 2;
         first = what == QG_MEAS_PLAQUETTE ? 0 : 2;
         return QG_OK;
     case QG_MEAS_PLAQUETTE_F32:
-        QG_CK(launch_plaquette_f32(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_results,
-                                   c->stream), "plaquette (FP32 products)");
+        QG_CK(launch_plaquette_f32(c->G, c->links, f.group, f.precision, c->d_params, tw, c->partials, c->d_ticket,
+                                   out, c->stream), "plaquette (FP32 products)");
         ncomp = 2;
-        first = 0;
         return QG_OK;
     case QG_MEAS_POLYAKOV:
-        QG_CK(launch_polyakov(c->G, c->links, f.group, f.precision, c->partials, c->d_results, c->stream), "polyakov");
+        QG_CK(launch_polyakov(c->G, c->links, f.group, f.precision, c->partials, c->d_ticket, out, c->stream),
+              "polyakov");
         ncomp = 4;
-        first = 0;
         return QG_OK;
     case QG_MEAS_WILSON:
         if (f.wilson_r < 1 || f.wilson_t < 1 || f.wilson_r > c->G.n[0] || f.wilson_t > c->G.n[3])
             return fail(c, QG_ERR_ARG, "Wilson loop extent out of range");
         QG_CK(launch_wilson(c->G, c->links, f.group, f.precision, f.wilson_r, f.wilson_t, c->d_params, tw, c->partials,
-                            c->d_results, c->stream), "wilson");
+                            c->d_ticket, out, c->stream), "wilson");
         ncomp = 1;
-        first = 0;
         return QG_OK;
     default:
         return fail(c, QG_ERR_ARG, "unknown measurement");
     }
+}
+
+extern "C" int qg_measure(qg_ctx *c, int what, double *out)
+{
+    if (!c || !out) return QG_ERR_ARG;
+    int ncomp = 0, first = 0;
+    int r = measure_launch(c, what, c->h_results, ncomp, first);
+    if (r) return r;
+    double v[4];
+    if ((r = measure_to_host(c, first + ncomp, v))) return r;
+    for (int i = 0; i < ncomp; i++) out[i] = v[first + i];
+    return QG_OK;
 }
 
 extern "C" int qg_measure_enqueue(qg_ctx *c, int what, uint64_t *ticket)
@@ -1583,13 +1563,11 @@ extern "C" int qg_measure_enqueue(qg_ctx *c, int what, uint64_t *ticket)
     if (!c || !ticket) return QG_ERR_ARG;
     const uint64_t t = c->ticket_next;
     const int slot = (int)(t % QG_MEASURE_SLOTS);
-    // the slot's previous copy must have landed before it is reused
+    // the slot's previous values must have landed before it is reused
     QG_CK(cudaEventSynchronize(c->ring_ev[slot]), "measure slot");
     int ncomp = 0, first = 0;
-    int r = measure_launch(c, what, ncomp, first);
+    int r = measure_launch(c, what, c->h_ring + 8 * slot, ncomp, first);
     if (r) return r;
-    QG_CK(cudaMemcpyAsync(c->h_ring + 8 * slot, c->d_results + first, ncomp * sizeof(double), cudaMemcpyDeviceToHost,
-                          c->stream), "measure copy");
     QG_CK(cudaEventRecord(c->ring_ev[slot], c->stream), "measure event");
     c->ring_ticket[slot] = t;
     c->ring_what[slot] = what;
@@ -1606,7 +1584,8 @@ extern "C" int qg_measure_fetch(qg_ctx *c, uint64_t ticket, double *out)
         return fail(c, QG_ERR_ARG, "unknown measurement ticket (never issued, or more than QG_MEASURE_SLOTS ago)");
     QG_CK(cudaEventSynchronize(c->ring_ev[slot]), "measure fetch");
     const int n = c->ring_what[slot] == QG_MEAS_POLYAKOV ? 4 : c->ring_what[slot] == QG_MEAS_WILSON ? 1 : 2;
-    for (int i = 0; i < n; i++) out[i] = c->h_ring[8 * slot + i];
+    const int first = c->ring_what[slot] == QG_MEAS_ACTION ? 2 : 0;
+    for (int i = 0; i < n; i++) out[i] = c->h_ring[8 * slot + first + i];
     return QG_OK;
 }
 

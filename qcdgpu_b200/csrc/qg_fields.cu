@@ -417,24 +417,24 @@ cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint
 // fold away at compile time
 template <int NC, typename Real, bool TW>
 __global__ void __launch_bounds__(256) k_plaquette(Field<Real> U, Geom G, const double *params, int twist,
-                                                    double *partials)
+                                                    double *partials, unsigned *ticket, double *out)
 {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     double v[4] = { 0, 0, 0, 0 };
     if (s < G.V) plaq_site<NC, Real>(U, G, params, TW ? twist : 0, s, v);
-    block_sum_store<4>(v, partials);
+    grid_sum<4, 256>(v, partials, ticket, out);
 }
 
 uint32_t plaq_blocks(const Geom &G) { return (G.V + 255) / 256; }
 
 cudaError_t launch_plaquette(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
-                             double *partials, double *out, cudaStream_t s)
+                             double *partials, unsigned *ticket, double *out, cudaStream_t s)
 {
     uint32_t nb = plaq_blocks(G);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-#define QG_PLQ(NC, R) (twist ? k_plaquette<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials) \
-                             : k_plaquette<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials))
+#define QG_PLQ(NC, R) (twist ? k_plaquette<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out) \
+                             : k_plaquette<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out))
         if (group == 3) QG_PLQ(3, double);
         else QG_PLQ(2, double);
     } else {
@@ -443,69 +443,64 @@ cudaError_t launch_plaquette(const Geom &G, const void *links, int group, int pr
         else QG_PLQ(2, float);
     }
 #undef QG_PLQ
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_reduce(partials, nb, 4, out, s);
+    return cudaGetLastError();
 }
 
 // the plaquette with FP32 products (QG_MEAS_PLAQUETTE_F32): same blocks,
 // partials and reduction as k_plaquette; FP64 links take k_plaquette
 template <int NC, bool TW>
 __global__ void __launch_bounds__(256) k_plaquette_f32(Field<float> U, Geom G, const double *params, int twist,
-                                                        double *partials)
+                                                        double *partials, unsigned *ticket, double *out)
 {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     double v[4] = { 0, 0, 0, 0 };
     if (s < G.V) plaq_site_f32<NC>(U, G, params, TW ? twist : 0, lex2crd(G, s), v);
-    block_sum_store<4>(v, partials);
+    grid_sum<4, 256>(v, partials, ticket, out);
 }
 
 cudaError_t launch_plaquette_f32(const Geom &G, const void *links, int group, int prec, const double *params,
-                                 int twist, double *partials, double *out, cudaStream_t s)
+                                 int twist, double *partials, unsigned *ticket, double *out, cudaStream_t s)
 {
-    if (prec) return launch_plaquette(G, links, group, prec, params, twist, partials, out, s);
+    if (prec) return launch_plaquette(G, links, group, prec, params, twist, partials, ticket, out, s);
     uint32_t nb = plaq_blocks(G);
     Field<float> U{ (float4 *)links, G.pstride };
     if (group == 3) {
-        if (twist) k_plaquette_f32<3, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials);
-        else k_plaquette_f32<3, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials);
+        if (twist) k_plaquette_f32<3, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
+        else k_plaquette_f32<3, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
     } else {
-        if (twist) k_plaquette_f32<2, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials);
-        else k_plaquette_f32<2, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials);
+        if (twist) k_plaquette_f32<2, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
+        else k_plaquette_f32<2, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_reduce(partials, nb, 4, out, s);
+    return cudaGetLastError();
 }
 
 // lattice_polyakov (polyakov.cl:54-140): one thread per spatial site
 template <int NC, typename Real>
-__global__ void __launch_bounds__(256) k_polyakov(Field<Real> U, Geom G, double *partials)
+__global__ void __launch_bounds__(256) k_polyakov(Field<Real> U, Geom G, double *partials, unsigned *ticket,
+                                                   double *out)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     double v[4] = { 0, 0, 0, 0 };
     if (i < (uint32_t)G.n[0] * G.n[1] * G.n[2]) poly_site<NC, Real>(U, G, i, v);
-    block_sum_store<4>(v, partials);
+    grid_sum<4, 256>(v, partials, ticket, out);
 }
 
 uint32_t poly_blocks(const Geom &G) { return ((uint32_t)G.n[0] * G.n[1] * G.n[2] + 255) / 256; }
 
-cudaError_t launch_polyakov(const Geom &G, const void *links, int group, int prec, double *partials, double *out,
-                            cudaStream_t s)
+cudaError_t launch_polyakov(const Geom &G, const void *links, int group, int prec, double *partials, unsigned *ticket,
+                            double *out, cudaStream_t s)
 {
     uint32_t nb = poly_blocks(G);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) k_polyakov<3, double><<<nb, 256, 0, s>>>(U, G, partials);
-        else k_polyakov<2, double><<<nb, 256, 0, s>>>(U, G, partials);
+        if (group == 3) k_polyakov<3, double><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
+        else k_polyakov<2, double><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
     } else {
         Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) k_polyakov<3, float><<<nb, 256, 0, s>>>(U, G, partials);
-        else k_polyakov<2, float><<<nb, 256, 0, s>>>(U, G, partials);
+        if (group == 3) k_polyakov<3, float><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
+        else k_polyakov<2, float><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_reduce(partials, nb, 4, out, s);
+    return cudaGetLastError();
 }
 
 // One-pass measurements: the per-site work once, the totals exactly as
@@ -515,7 +510,7 @@ cudaError_t launch_polyakov(const Geom &G, const void *links, int group, int pre
 // qg_measure / qg_measure_*_profile calls bit for bit.
 template <int NC, typename Real, bool TW>
 __global__ void __launch_bounds__(256) k_plaq_sites(Field<Real> U, Geom G, const double *params, int twist,
-                                                     double *partials, double *sites)
+                                                     double *partials, unsigned *ticket, double *out, double *sites)
 {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     double v[4] = { 0, 0, 0, 0 };
@@ -524,10 +519,11 @@ __global__ void __launch_bounds__(256) k_plaq_sites(Field<Real> U, Geom G, const
         sites[s] = v[2];                                 // spatial action of the site
         sites[(size_t)G.V + s] = v[3];                   // temporal
     }
-    block_sum_store<4>(v, partials);
+    grid_sum<4, 256>(v, partials, ticket, out);
 }
 template <int NC, typename Real>
-__global__ void __launch_bounds__(256) k_poly_sites(Field<Real> U, Geom G, double *partials, double *sites)
+__global__ void __launch_bounds__(256) k_poly_sites(Field<Real> U, Geom G, double *partials, unsigned *ticket,
+                                                     double *out, double *sites)
 {
     const uint32_t Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -537,7 +533,7 @@ __global__ void __launch_bounds__(256) k_poly_sites(Field<Real> U, Geom G, doubl
         sites[i] = v[0];
         sites[(size_t)Vs + i] = v[1];
     }
-    block_sum_store<4>(v, partials);
+    grid_sum<4, 256>(v, partials, ticket, out);
 }
 // k_profile's loop over the stored site values (KIND 0: action per lattice
 // site, lexicographic index; KIND 1: Polyakov trace per spatial site,
@@ -564,33 +560,32 @@ __global__ void __launch_bounds__(256) k_bin_sites(const double *sites, Geom G, 
 // 712-1175 and reduce_measurement_plq_double2 :1313-1357): 12 sums
 template <int NC, typename Real, bool TW>
 __global__ void __launch_bounds__(256) k_fmunu(Field<Real> U, Geom G, const double *params, int twist, int field,
-                                                int i1, int i2, double *partials)
+                                                int i1, int i2, double *partials, unsigned *ticket, double *out)
 {
     if (!TW) twist = 0;                  // untwisted: the twist tests fold away
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     double v[12] = { 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0 };
     if (s < G.V) fmunu_site<NC, Real>(U, G, params, twist, s, field, i1, i2, v);
-    block_sum_store<12>(v, partials);
+    grid_sum<12, 256>(v, partials, ticket, out);
 }
 
 uint32_t fmunu_partials(const Geom &G) { return plaq_blocks(G) * 12; }
 
 cudaError_t launch_fmunu(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
-                         int field, int i1, int i2, double *partials, double *out, cudaStream_t s)
+                         int field, int i1, int i2, double *partials, unsigned *ticket, double *out,
+                         cudaStream_t s)
 {
     uint32_t nb = plaq_blocks(G);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) (twist ? k_fmunu<3, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials) : k_fmunu<3, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials));
-        else (twist ? k_fmunu<2, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials) : k_fmunu<2, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials));
+        if (group == 3) (twist ? k_fmunu<3, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<3, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
+        else (twist ? k_fmunu<2, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<2, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
     } else {
         Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) (twist ? k_fmunu<3, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials) : k_fmunu<3, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials));
-        else (twist ? k_fmunu<2, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials) : k_fmunu<2, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials));
+        if (group == 3) (twist ? k_fmunu<3, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<3, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
+        else (twist ? k_fmunu<2, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<2, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_reduce(partials, nb, 12, out, s);
+    return cudaGetLastError();
 }
 
 // Profiles along x, y or z (lattice_action_diff_{x,y,z},
@@ -678,8 +673,8 @@ cudaError_t launch_profile(const Geom &G, const void *links, int group, int prec
 size_t sites_buffer_doubles(const Geom &G) { return 2 * (size_t)G.V; }
 
 cudaError_t launch_measure_all(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
-                               int kind, double *partials, double *ppartials, double *sites, double *out,
-                               cudaStream_t s)
+                               int kind, double *partials, double *ppartials, double *sites, unsigned *ticket,
+                               double *out, cudaStream_t s)
 {
     // totals into out[0..3], site values into `sites`
     const uint32_t Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
@@ -687,16 +682,15 @@ cudaError_t launch_measure_all(const Geom &G, const void *links, int group, int 
 #define QG_SITES(NC, R)                                                                                 \
     do {                                                                                                \
         Field<R> U{ (typename V4<R>::T *)links, G.pstride };                                            \
-        if (kind == 0 && twist) k_plaq_sites<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, sites); \
-        else if (kind == 0) k_plaq_sites<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, sites); \
-        else k_poly_sites<NC, R><<<nb, 256, 0, s>>>(U, G, partials, sites);                            \
+        if (kind == 0 && twist) k_plaq_sites<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out, sites); \
+        else if (kind == 0) k_plaq_sites<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out, sites); \
+        else k_poly_sites<NC, R><<<nb, 256, 0, s>>>(U, G, partials, ticket, out, sites);                            \
     } while (0)
     if (prec) { if (group == 3) QG_SITES(3, double); else QG_SITES(2, double); }
     else { if (group == 3) QG_SITES(3, float); else QG_SITES(2, float); }
 #undef QG_SITES
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if ((e = launch_reduce(partials, nb, 4, out, s)) != cudaSuccess) return e;
     // per-slice sums along x, y, z into out[4 ..]
     double *o = out + 4;
     for (int axis = 0; axis < 3; axis++) {
@@ -716,7 +710,7 @@ cudaError_t launch_measure_all(const Geom &G, const void *links, int group, int 
 // {x,y,z}, Re Tr(L_t^T(x) L_i^R(x+T t) L_t^T(x+R i)^+ L_i^R(x)^+) in FP64
 template <int NC, typename Real, bool TW>
 __global__ void __launch_bounds__(128) k_wilson(Field<Real> U, Geom G, int R, int T, const double *params, int twist,
-                                                 double *partials)
+                                                 double *partials, unsigned *ticket, double *out)
 {
     if (!TW) twist = 0;                  // untwisted: the twist tests fold away
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -744,25 +738,23 @@ __global__ void __launch_bounds__(128) k_wilson(Field<Real> U, Geom G, int R, in
         }
         v[0] = acc;
     }
-    block_sum_store<1>(v, partials);
+    grid_sum<1, 128>(v, partials, ticket, out);
 }
 
 cudaError_t launch_wilson(const Geom &G, const void *links, int group, int prec, int R, int T, const double *params,
-                          int twist, double *partials, double *out, cudaStream_t s)
+                          int twist, double *partials, unsigned *ticket, double *out, cudaStream_t s)
 {
     uint32_t nb = (G.V + 127) / 128;
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) (twist ? k_wilson<3, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials) : k_wilson<3, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials));
-        else (twist ? k_wilson<2, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials) : k_wilson<2, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials));
+        if (group == 3) (twist ? k_wilson<3, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<3, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
+        else (twist ? k_wilson<2, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<2, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
     } else {
         Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) (twist ? k_wilson<3, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials) : k_wilson<3, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials));
-        else (twist ? k_wilson<2, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials) : k_wilson<2, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials));
+        if (group == 3) (twist ? k_wilson<3, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<3, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
+        else (twist ? k_wilson<2, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<2, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_reduce(partials, nb, 1, out, s);
+    return cudaGetLastError();
 }
 
 // All planar Wilson loops R x T, R <= Rmax, T <= Tmax (<= 16), in one
@@ -967,18 +959,6 @@ cudaError_t launch_wilson_all(const Geom &G, const void *links, int group, int p
     }
     if (e != cudaSuccess) return e;
     k_wilson_all_reduce<<<(Rmax * Tmax + 127) / 128, 128, 0, s>>>(partials, nbx, Rmax, Tmax, out);
-    return cudaGetLastError();
-}
-
-// final pass: one block sums the partials in a fixed order (deterministic)
-__global__ void __launch_bounds__(1024) k_reduce(const double *partials, uint32_t nblocks, int ncomp, double *out)
-{
-    reduce_partials(partials, nblocks, ncomp, out);
-}
-
-cudaError_t launch_reduce(const double *partials, uint32_t nblocks, int ncomp, double *out, cudaStream_t s)
-{
-    k_reduce<<<1, 1024, 0, s>>>(partials, nblocks, ncomp, out);
     return cudaGetLastError();
 }
 

@@ -52,24 +52,25 @@ void ref_stage_free(RefStage &st);
 cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
                            RefStage &st, cudaStream_t s);
 
-// measurements: per-block partials into scratch, then a fixed-order final
-// reduction into out (device).  Partials sizes returned by *_blocks().
+// measurements: per-block partials into scratch, summed in a fixed order by
+// the last block into out (device or page-locked host memory); *ticket is a
+// zeroed device counter that concurrent launches do not share.  Partials
+// sizes returned by *_blocks().
 uint32_t plaq_blocks(const Geom &G);
 cudaError_t launch_plaquette(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
-                             double *partials, double *out, cudaStream_t s);
+                             double *partials, unsigned *ticket, double *out, cudaStream_t s);
 // the plaquette with FP32 products on FP32 links (as launch_plaquette on FP64 links)
 cudaError_t launch_plaquette_f32(const Geom &G, const void *links, int group, int prec, const double *params,
-                                 int twist, double *partials, double *out, cudaStream_t s);
+                                 int twist, double *partials, unsigned *ticket, double *out, cudaStream_t s);
 uint32_t poly_blocks(const Geom &G);
-cudaError_t launch_polyakov(const Geom &G, const void *links, int group, int prec, double *partials, double *out,
-                            cudaStream_t s);
+cudaError_t launch_polyakov(const Geom &G, const void *links, int group, int prec, double *partials, unsigned *ticket,
+                            double *out, cudaStream_t s);
 cudaError_t launch_wilson(const Geom &G, const void *links, int group, int prec, int R, int T, const double *params,
-                          int twist, double *partials, double *out, cudaStream_t s);
-cudaError_t launch_reduce(const double *partials, uint32_t nblocks, int ncomp, double *out, cudaStream_t s);
+                          int twist, double *partials, unsigned *ticket, double *out, cudaStream_t s);
 // F_munu sums (12) of the plaquettes of field 0 (xy,xz,yz) / 1 (xt,yt,zt)
 uint32_t fmunu_partials(const Geom &G);
 cudaError_t launch_fmunu(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
-                         int field, int i1, int i2, double *partials, double *out, cudaStream_t s);
+                         int field, int i1, int i2, double *partials, unsigned *ticket, double *out, cudaStream_t s);
 // per-slice sums along axis 0..2: kind 0 action (spatial, temporal), kind 1
 // Polyakov trace (Re, Im); out holds 2 n[axis] doubles
 uint32_t profile_partials(const Geom &G);
@@ -79,8 +80,8 @@ uint32_t profile_partials(const Geom &G);
 // sites_buffer_doubles(G)
 size_t sites_buffer_doubles(const Geom &G);
 cudaError_t launch_measure_all(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
-                               int kind, double *partials, double *ppartials, double *sites, double *out,
-                               cudaStream_t s);
+                               int kind, double *partials, double *ppartials, double *sites, unsigned *ticket,
+                               double *out, cudaStream_t s);
 cudaError_t launch_profile(const Geom &G, const void *links, int group, int prec, const double *params, int twist,
                            int kind, int axis, double *partials, double *out, cudaStream_t s);
 int wilson_all_blocks(const Geom &G);

@@ -340,4 +340,58 @@ __device__ __forceinline__ void reduce_partials(const double *partials, uint32_t
     }
 }
 
+// Block sums and the whole grid's sums in one launch: the block that takes
+// the last ticket sums the partials as reduce_partials does with 1024
+// threads (each thread stands for 1024 / THREADS of them), so the result has
+// the bits of the two-launch form, and writes it to out -- which may be
+// page-locked host memory: the launch of the second pass (4 us of a 25 us
+// measurement at 8^4) and the copy of the result go.  *ticket is zero
+// before and after.
+template <int K, int THREADS>
+__device__ __forceinline__ void grid_sum(double (&v)[K], double *partials, unsigned *ticket, double *out)
+{
+    block_sum_store<K>(v, partials);
+    __shared__ unsigned s_last;
+    if (threadIdx.x == 0) {                              // the thread that wrote the block's partials
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) + 1u == gridDim.x;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    constexpr int NV = 1024 / THREADS, KC = K < 4 ? K : 4;
+    __shared__ double sh[K][32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t n = gridDim.x;
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += KC) {
+        double x[KC][NV];
+#pragma unroll
+        for (int k = 0; k < KC; k++)
+#pragma unroll
+            for (int j = 0; j < NV; j++) x[k][j] = 0;
+        for (uint32_t b = tid; b < n; b += 1024)
+#pragma unroll
+            for (int j = 0; j < NV; j++)
+                if (b + j * THREADS < n)
+#pragma unroll
+                    for (int k = 0; k < KC; k++) x[k][j] += __ldcg(partials + (size_t)(b + j * THREADS) * K + k0 + k);
+#pragma unroll
+        for (int k = 0; k < KC; k++)
+#pragma unroll
+            for (int j = 0; j < NV; j++) {
+                double y = x[k][j];
+                for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+                if (lane == 0) sh[k0 + k][j * (THREADS / 32) + wid] = y;
+            }
+    }
+    __syncthreads();
+    for (int k = wid; k < K; k += THREADS / 32) {
+        double y = sh[k][lane];
+        for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+        if (lane == 0) out[k] = y;
+    }
+    if (tid == 0) *ticket = 0;
+}
+
 }  // namespace qg
