@@ -410,6 +410,21 @@ cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint
     return cudaSuccess;
 }
 
+// final pass: one block sums the partials in a fixed order (deterministic)
+__global__ void __launch_bounds__(1024) k_reduce(const double *partials, uint32_t nblocks, int ncomp, double *out)
+{
+    reduce_partials(partials, nblocks, ncomp, out);
+}
+
+// the sum of a measurement's partials: in its own launch (grid_sum) while its
+// blocks are about one wave, else by k_reduce; the same bits
+static unsigned *fused_ticket(uint32_t nb, unsigned *ticket) { return nb <= 4 * 148 ? ticket : nullptr; }
+static cudaError_t finish_sum(uint32_t nb, int ncomp, const double *partials, double *out, cudaStream_t s)
+{
+    if (!fused_ticket(nb, (unsigned *)1)) k_reduce<<<1, 1024, 0, s>>>(partials, nb, ncomp, out);
+    return cudaGetLastError();
+}
+
 // ------------------------------------------------------------ observables
 // lattice_measurement_plq + lattice_measurement (sun_measurements_cl.cl:
 // 55-184,1178-1311): per-site plaquette and action sums, block partials
@@ -431,10 +446,11 @@ cudaError_t launch_plaquette(const Geom &G, const void *links, int group, int pr
                              double *partials, unsigned *ticket, double *out, cudaStream_t s)
 {
     uint32_t nb = plaq_blocks(G);
+    unsigned *tk = fused_ticket(nb, ticket);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-#define QG_PLQ(NC, R) (twist ? k_plaquette<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out) \
-                             : k_plaquette<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out))
+#define QG_PLQ(NC, R) (twist ? k_plaquette<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out) \
+                             : k_plaquette<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out))
         if (group == 3) QG_PLQ(3, double);
         else QG_PLQ(2, double);
     } else {
@@ -443,7 +459,7 @@ cudaError_t launch_plaquette(const Geom &G, const void *links, int group, int pr
         else QG_PLQ(2, float);
     }
 #undef QG_PLQ
-    return cudaGetLastError();
+    return finish_sum(nb, 4, partials, out, s);
 }
 
 // the plaquette with FP32 products (QG_MEAS_PLAQUETTE_F32): same blocks,
@@ -463,15 +479,16 @@ cudaError_t launch_plaquette_f32(const Geom &G, const void *links, int group, in
 {
     if (prec) return launch_plaquette(G, links, group, prec, params, twist, partials, ticket, out, s);
     uint32_t nb = plaq_blocks(G);
+    unsigned *tk = fused_ticket(nb, ticket);
     Field<float> U{ (float4 *)links, G.pstride };
     if (group == 3) {
-        if (twist) k_plaquette_f32<3, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
-        else k_plaquette_f32<3, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
+        if (twist) k_plaquette_f32<3, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out);
+        else k_plaquette_f32<3, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out);
     } else {
-        if (twist) k_plaquette_f32<2, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
-        else k_plaquette_f32<2, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out);
+        if (twist) k_plaquette_f32<2, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out);
+        else k_plaquette_f32<2, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out);
     }
-    return cudaGetLastError();
+    return finish_sum(nb, 4, partials, out, s);
 }
 
 // lattice_polyakov (polyakov.cl:54-140): one thread per spatial site
@@ -491,16 +508,17 @@ cudaError_t launch_polyakov(const Geom &G, const void *links, int group, int pre
                             double *out, cudaStream_t s)
 {
     uint32_t nb = poly_blocks(G);
+    unsigned *tk = fused_ticket(nb, ticket);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) k_polyakov<3, double><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
-        else k_polyakov<2, double><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
+        if (group == 3) k_polyakov<3, double><<<nb, 256, 0, s>>>(U, G, partials, tk, out);
+        else k_polyakov<2, double><<<nb, 256, 0, s>>>(U, G, partials, tk, out);
     } else {
         Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) k_polyakov<3, float><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
-        else k_polyakov<2, float><<<nb, 256, 0, s>>>(U, G, partials, ticket, out);
+        if (group == 3) k_polyakov<3, float><<<nb, 256, 0, s>>>(U, G, partials, tk, out);
+        else k_polyakov<2, float><<<nb, 256, 0, s>>>(U, G, partials, tk, out);
     }
-    return cudaGetLastError();
+    return finish_sum(nb, 4, partials, out, s);
 }
 
 // One-pass measurements: the per-site work once, the totals exactly as
@@ -576,16 +594,17 @@ cudaError_t launch_fmunu(const Geom &G, const void *links, int group, int prec, 
                          cudaStream_t s)
 {
     uint32_t nb = plaq_blocks(G);
+    unsigned *tk = fused_ticket(nb, ticket);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) (twist ? k_fmunu<3, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<3, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
-        else (twist ? k_fmunu<2, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<2, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
+        if (group == 3) (twist ? k_fmunu<3, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out) : k_fmunu<3, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out));
+        else (twist ? k_fmunu<2, double, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out) : k_fmunu<2, double, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out));
     } else {
         Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) (twist ? k_fmunu<3, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<3, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
-        else (twist ? k_fmunu<2, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out) : k_fmunu<2, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, ticket, out));
+        if (group == 3) (twist ? k_fmunu<3, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out) : k_fmunu<3, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out));
+        else (twist ? k_fmunu<2, float, true><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out) : k_fmunu<2, float, false><<<nb, 256, 0, s>>>(U, G, params, twist, field, i1, i2, partials, tk, out));
     }
-    return cudaGetLastError();
+    return finish_sum(nb, 12, partials, out, s);
 }
 
 // Profiles along x, y or z (lattice_action_diff_{x,y,z},
@@ -679,17 +698,18 @@ cudaError_t launch_measure_all(const Geom &G, const void *links, int group, int 
     // totals into out[0..3], site values into `sites`
     const uint32_t Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
     const uint32_t nb = kind == 0 ? plaq_blocks(G) : (Vs + 255) / 256;
+    unsigned *tk = fused_ticket(nb, ticket);
 #define QG_SITES(NC, R)                                                                                 \
     do {                                                                                                \
         Field<R> U{ (typename V4<R>::T *)links, G.pstride };                                            \
-        if (kind == 0 && twist) k_plaq_sites<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out, sites); \
-        else if (kind == 0) k_plaq_sites<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, ticket, out, sites); \
-        else k_poly_sites<NC, R><<<nb, 256, 0, s>>>(U, G, partials, ticket, out, sites);                            \
+        if (kind == 0 && twist) k_plaq_sites<NC, R, true><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out, sites); \
+        else if (kind == 0) k_plaq_sites<NC, R, false><<<nb, 256, 0, s>>>(U, G, params, twist, partials, tk, out, sites); \
+        else k_poly_sites<NC, R><<<nb, 256, 0, s>>>(U, G, partials, tk, out, sites);                            \
     } while (0)
     if (prec) { if (group == 3) QG_SITES(3, double); else QG_SITES(2, double); }
     else { if (group == 3) QG_SITES(3, float); else QG_SITES(2, float); }
 #undef QG_SITES
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = finish_sum(nb, 4, partials, out, s);
     if (e != cudaSuccess) return e;
     // per-slice sums along x, y, z into out[4 ..]
     double *o = out + 4;
@@ -745,16 +765,17 @@ cudaError_t launch_wilson(const Geom &G, const void *links, int group, int prec,
                           int twist, double *partials, unsigned *ticket, double *out, cudaStream_t s)
 {
     uint32_t nb = (G.V + 127) / 128;
+    unsigned *tk = fused_ticket(nb, ticket);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) (twist ? k_wilson<3, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<3, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
-        else (twist ? k_wilson<2, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<2, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
+        if (group == 3) (twist ? k_wilson<3, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<3, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
+        else (twist ? k_wilson<2, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<2, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
     } else {
         Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) (twist ? k_wilson<3, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<3, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
-        else (twist ? k_wilson<2, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out) : k_wilson<2, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, ticket, out));
+        if (group == 3) (twist ? k_wilson<3, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<3, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
+        else (twist ? k_wilson<2, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<2, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
     }
-    return cudaGetLastError();
+    return finish_sum(nb, 1, partials, out, s);
 }
 
 // All planar Wilson loops R x T, R <= Rmax, T <= Tmax (<= 16), in one

@@ -92,6 +92,32 @@ __device__ __forceinline__ double retr4(const M3<double> &a, const M3<double> &b
     return tr;
 }
 
+// SU(2) links as the quaternions they are stored as (x + i z, y + i w; -y + i w,
+// x - i z), in FP64: a product is 16 multiply-adds, embedded in 3 x 3 it is 108
+template <typename Real>
+__device__ __forceinline__ R4<double> load_q(const Field<Real> &U, const Geom &G, const Crd &c, int mu,
+                                             const double *params, int twist)
+{
+    R4<Real> m = U.ldg2(mu, cb_index(G, c, parity_of(c)));
+    if (twist && mu == 1 && c.x == G.n[0] - 1) {
+        Real ph = param_real<Real>(params[1]);
+        R4<Real> om = { RC<Real>::cs(ph / 2), 0, RC<Real>::sn(ph / 2), 0 };
+        m = times2(om, m);
+    }
+    return { (double)m.x, (double)m.y, (double)m.z, (double)m.w };
+}
+// Re Tr(a b c^+ d^+) = 2 (a b) . (d c)
+__device__ __forceinline__ double retr4q(const R4<double> &a, const R4<double> &b, const R4<double> &c,
+                                         const R4<double> &d)
+{
+    const R4<double> p = times2(a, b), q = times2(d, c);
+    double tr = p.x * q.x;
+    tr = FMA(p.y, q.y, tr);
+    tr = FMA(p.z, q.z, tr);
+    tr = FMA(p.w, q.w, tr);
+    return 2.0 * tr;
+}
+
 // warp + block sum of K doubles; thread 0 writes the block's partials
 template <int K>
 __device__ __forceinline__ void block_sum_store(double (&v)[K], double *partials, uint32_t block = 0xffffffffu)
@@ -124,18 +150,23 @@ __device__ __forceinline__ void plaq_site_c(const Field<Real> &U, const Geom &G,
                                             const Crd &c, double (&v)[4])
 {
     const Crd cx = step_plus(G, c, 0), cy = step_plus(G, c, 1), cz = step_plus(G, c, 2), ct = step_plus(G, c, 3);
-    M3<double> m1 = load_d<NC, Real>(U, G, c, 0, params, twist);
-    M3<double> m4 = load_d<NC, Real>(U, G, c, 1, params, twist);
-    M3<double> m5 = load_d<NC, Real>(U, G, c, 2, params, twist);
-    M3<double> m6 = load_d<NC, Real>(U, G, c, 3, params, twist);
     const double bet = (double)param_real<Real>(params[0]);
     double rs, rt;
-    rs  = retr4(m1, load_d<NC, Real>(U, G, cx, 1, params, twist), load_d<NC, Real>(U, G, cy, 0, params, twist), m4);
-    rs += retr4(m1, load_d<NC, Real>(U, G, cx, 2, params, twist), load_d<NC, Real>(U, G, cz, 0, params, twist), m5);
-    rt  = retr4(m1, load_d<NC, Real>(U, G, cx, 3, params, twist), load_d<NC, Real>(U, G, ct, 0, params, twist), m6);
-    rs += retr4(m4, load_d<NC, Real>(U, G, cy, 2, params, twist), load_d<NC, Real>(U, G, cz, 1, params, twist), m5);
-    rt += retr4(m4, load_d<NC, Real>(U, G, cy, 3, params, twist), load_d<NC, Real>(U, G, ct, 1, params, twist), m6);
-    rt += retr4(m5, load_d<NC, Real>(U, G, cz, 3, params, twist), load_d<NC, Real>(U, G, ct, 2, params, twist), m6);
+    auto planes = [&](auto ld, auto retr) {
+        const auto m1 = ld(c, 0), m4 = ld(c, 1), m5 = ld(c, 2), m6 = ld(c, 3);
+        rs  = retr(m1, ld(cx, 1), ld(cy, 0), m4);
+        rs += retr(m1, ld(cx, 2), ld(cz, 0), m5);
+        rt  = retr(m1, ld(cx, 3), ld(ct, 0), m6);
+        rs += retr(m4, ld(cy, 2), ld(cz, 1), m5);
+        rt += retr(m4, ld(cy, 3), ld(ct, 1), m6);
+        rt += retr(m5, ld(cz, 3), ld(ct, 2), m6);
+    };
+    if constexpr (NC == 3)
+        planes([&](const Crd &q, int mu) { return load_d<NC, Real>(U, G, q, mu, params, twist); },
+               [](const M3<double> &a, const M3<double> &b, const M3<double> &e, const M3<double> &f) { return retr4(a, b, e, f); });
+    else
+        planes([&](const Crd &q, int mu) { return load_q<Real>(U, G, q, mu, params, twist); },
+               [](const R4<double> &a, const R4<double> &b, const R4<double> &e, const R4<double> &f) { return retr4q(a, b, e, f); });
     v[0] = rs; v[1] = rt;
     v[2] = bet * (3.0 * NC - rs);
     v[3] = bet * (3.0 * NC - rt);
@@ -179,10 +210,15 @@ __device__ __forceinline__ void poly_site_c(const Field<Real> &U, const Geom &G,
     double pr, pi;
     c.t = 0;
     if (NC == 3) {
-        M3<Real> v0 = expand(U.ldg3(3, cb_index(G, c, parity_of(c))));
+        // two links ahead are loaded under a product: the columns are few and
+        // their chains of N4 products long (32^4: FP32 36 -> 30, FP64 57 -> 38 us)
+        auto at = [&](int k) { c.t = k < G.n[3] ? k : 0; return U.ldg3(3, cb_index(G, c, parity_of(c))); };
+        M3<Real> v0 = expand(at(0));
+        G3<Real> n1 = at(1), n2 = at(2);
         for (int k = 1; k < G.n[3]; k++) {
-            c.t = k;
-            M3<Real> v1 = expand(U.ldg3(3, cb_index(G, c, parity_of(c))));
+            const M3<Real> v1 = expand(n1);
+            n1 = n2;
+            n2 = at(k + 2);
             v0 = mulf(v0, v1);
         }
         pr = (double)v0.m[0][0].re + (double)v0.m[1][1].re + (double)v0.m[2][2].re;
@@ -231,21 +267,17 @@ __device__ __forceinline__ M3<double> plaq_matrix(const M3<double> &a, const M3<
     return r;
 }
 
-// -i Tr(P T_a): T_a = lambda_a / 2 (SU(3), a = 1..8; trace_lambda1..8_double,
-// su3_measurements_cl.cl:355-460) or sigma_a / 2 (SU(2), a = 1..3, real
-// part only; trace_sigma1..3_double, su2_measurements_cl.cl:89-124) -- the
-// generator's two (three) non-zero entries picked out of P
-template <int NC>
+// -i Tr(P T_a), T_a = lambda_a / 2 (SU(3), a = 1..8; trace_lambda1..8_double,
+// su3_measurements_cl.cl:355-460): the generator's two (three) non-zero
+// entries picked out of P.  (SU(2), sigma_a / 2, a = 1..3, real part only;
+// trace_sigma1..3_double, su2_measurements_cl.cl:89-124: a component of the
+// plaquette's quaternion, fmunu_site)
 __device__ __forceinline__ void gen_proj(const M3<double> &P, int a, double &re, double &im)
 {
     const CX<double> u1 = P.m[0][0], u2 = P.m[0][1], u3 = P.m[0][2];
     const CX<double> v1 = P.m[1][0], v2 = P.m[1][1], v3 = P.m[1][2];
     const CX<double> w1 = P.m[2][0], w2 = P.m[2][1], w3 = P.m[2][2];
     re = 0; im = 0;
-    if (NC == 2) {
-        re = a == 1 ? u2.im : a == 2 ? u2.re : u1.im;
-        return;
-    }
     switch (a) {
     case 1: re = u2.im + v1.im; im = -u2.re - v1.re; break;
     case 2: re = u2.re - v1.re; im = u2.im - v1.im; break;
@@ -275,14 +307,22 @@ __device__ __forceinline__ void fmunu_site(const Field<Real> &U, const Geom &G, 
         const int m = field ? p : (p == 2 ? 1 : 0);
         const int n = field ? 3 : (p == 0 ? 1 : 2);
         const Crd cm = step_plus(G, c, m), cn = step_plus(G, c, n);
+        if constexpr (NC == 2) {
+            auto ld = [&](const Crd &q, int mu) { return load_q<Real>(U, G, q, mu, params, twist); };
+            const R4<double> P = times2(times2(ld(c, m), ld(cm, n)), herm2(times2(ld(c, n), ld(cn, m))));
+            auto proj = [&](int g) { return g == 1 ? P.w : g == 2 ? P.y : P.z; };
+            v[2 * p] = proj(i1); v[2 * p + 1] = 0;
+            v[6 + 2 * p] = proj(i2); v[7 + 2 * p] = 0;
+            continue;
+        }
         const M3<double> P = plaq_matrix(load_d<NC, Real>(U, G, c, m, params, twist),
                                          load_d<NC, Real>(U, G, cm, n, params, twist),
                                          load_d<NC, Real>(U, G, cn, m, params, twist),
                                          load_d<NC, Real>(U, G, c, n, params, twist));
         double re, im;
-        gen_proj<NC>(P, i1, re, im);
+        gen_proj(P, i1, re, im);
         v[2 * p] = re; v[2 * p + 1] = im;
-        gen_proj<NC>(P, i2, re, im);
+        gen_proj(P, i2, re, im);
         v[6 + 2 * p] = re; v[7 + 2 * p] = im;
     }
 }
@@ -346,11 +386,15 @@ __device__ __forceinline__ void reduce_partials(const double *partials, uint32_t
 // the bits of the two-launch form, and writes it to out -- which may be
 // page-locked host memory: the launch of the second pass (4 us of a 25 us
 // measurement at 8^4) and the copy of the result go.  *ticket is zero
-// before and after.
+// before and after.  A null ticket leaves the sum to a second launch: with
+// many blocks each one's wait for its ticket (a fence and an atomic, about
+// a microsecond with its registers held) costs more than that launch (32^4
+// plaquette, 4096 blocks: 238 against 221 us).
 template <int K, int THREADS>
 __device__ __forceinline__ void grid_sum(double (&v)[K], double *partials, unsigned *ticket, double *out)
 {
     block_sum_store<K>(v, partials);
+    if (!ticket) return;
     __shared__ unsigned s_last;
     if (threadIdx.x == 0) {                              // the thread that wrote the block's partials
         __threadfence();
