@@ -555,14 +555,19 @@ __global__ void __launch_bounds__(256) k_poly_sites(Field<Real> U, Geom G, doubl
 }
 // k_profile's loop over the stored site values (KIND 0: action per lattice
 // site, lexicographic index; KIND 1: Polyakov trace per spatial site,
-// i = y + N2 (z + N3 x))
+// i = y + N2 (z + N3 x)), all three axes in one launch: axis a's blocks are
+// [first[a], first[a + 1]), its slices' chunks in order
+struct Bins {
+    uint32_t first[4], per_slice[3], chunks[3];
+};
 template <int KIND>
-__global__ void __launch_bounds__(256) k_bin_sites(const double *sites, Geom G, int axis, uint32_t per_slice,
-                                                    uint32_t chunks, double *partials)
+__global__ void __launch_bounds__(256) k_bin_sites(const double *sites, Geom G, Bins B, double *partials)
 {
-    const int k = (int)(blockIdx.x / chunks);
-    const uint32_t j0 = (blockIdx.x % chunks) * 1024u;
-    const uint32_t j1 = min(per_slice, j0 + 1024u);
+    const int axis = blockIdx.x >= B.first[2] ? 2 : blockIdx.x >= B.first[1] ? 1 : 0;
+    const uint32_t chunks = B.chunks[axis], b = blockIdx.x - B.first[axis];
+    const int k = (int)(b / chunks);
+    const uint32_t j0 = (b % chunks) * 1024u;
+    const uint32_t j1 = min(B.per_slice[axis], j0 + 1024u);
     const size_t n = KIND == 0 ? (size_t)G.V : (size_t)G.n[0] * G.n[1] * G.n[2];
     double acc[2] = { 0, 0 };
     for (uint32_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
@@ -572,6 +577,13 @@ __global__ void __launch_bounds__(256) k_bin_sites(const double *sites, Geom G, 
         acc[1] += sites[n + s];
     }
     block_sum_store<2>(acc, partials);
+}
+// block = slice (x, then y, then z slices): the sum of its chunks
+__global__ void __launch_bounds__(256) k_bin_reduce(const double *partials, Geom G, Bins B, double *out)
+{
+    const int q = blockIdx.x, axis = q >= G.n[0] + G.n[1] ? 2 : q >= G.n[0] ? 1 : 0;
+    const int k = q - (axis == 2 ? G.n[0] + G.n[1] : axis == 1 ? G.n[0] : 0);
+    reduce_partials(partials + ((size_t)B.first[axis] + (size_t)k * B.chunks[axis]) * 2, B.chunks[axis], 2, out + 2 * q);
 }
 
 // F_munu (FMUNU / F0MU lattice_measurement_plq, sun_measurements_cl.cl:
@@ -648,16 +660,19 @@ static uint32_t profile_per_slice(const Geom &G, int axis, int kind)
     uint32_t n = (uint32_t)G.n[0] * G.n[1] * G.n[2] * (kind == 0 ? G.n[3] : 1);
     return n / (uint32_t)G.n[axis];
 }
-uint32_t profile_partials(const Geom &G)
+static Bins profile_bins(const Geom &G, int kind)
 {
-    uint32_t m = 0;
-    for (int axis = 0; axis < 3; axis++)
-        for (int kind = 0; kind < 2; kind++) {
-            uint32_t chunks = (profile_per_slice(G, axis, kind) + kProfileChunk - 1) / kProfileChunk;
-            m = max(m, chunks * (uint32_t)G.n[axis] * 2);
-        }
-    return m;
+    Bins B;
+    B.first[0] = 0;
+    for (int a = 0; a < 3; a++) {
+        B.per_slice[a] = profile_per_slice(G, a, kind);
+        B.chunks[a] = (B.per_slice[a] + kProfileChunk - 1) / kProfileChunk;
+        B.first[a + 1] = B.first[a] + B.chunks[a] * (uint32_t)G.n[a];
+    }
+    return B;
 }
+// the three axes' partials side by side (the action's are the more)
+uint32_t profile_partials(const Geom &G) { return 2 * profile_bins(G, 0).first[3]; }
 
 template <int NC, typename Real>
 static void profile_kernel(int kind, uint32_t nb, const Field<Real> &U, const Geom &G, const double *params,
@@ -712,18 +727,11 @@ cudaError_t launch_measure_all(const Geom &G, const void *links, int group, int 
     cudaError_t e = finish_sum(nb, 4, partials, out, s);
     if (e != cudaSuccess) return e;
     // per-slice sums along x, y, z into out[4 ..]
-    double *o = out + 4;
-    for (int axis = 0; axis < 3; axis++) {
-        const uint32_t per = profile_per_slice(G, axis, kind);
-        const uint32_t chunks = (per + kProfileChunk - 1) / kProfileChunk;
-        const uint32_t nbk = chunks * (uint32_t)G.n[axis];
-        if (kind == 0) k_bin_sites<0><<<nbk, 256, 0, s>>>(sites, G, axis, per, chunks, ppartials);
-        else k_bin_sites<1><<<nbk, 256, 0, s>>>(sites, G, axis, per, chunks, ppartials);
-        k_profile_reduce<<<G.n[axis], 256, 0, s>>>(ppartials, chunks, o);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        o += 2 * G.n[axis];
-    }
-    return cudaSuccess;
+    const Bins B = profile_bins(G, kind);
+    if (kind == 0) k_bin_sites<0><<<B.first[3], 256, 0, s>>>(sites, G, B, ppartials);
+    else k_bin_sites<1><<<B.first[3], 256, 0, s>>>(sites, G, B, ppartials);
+    k_bin_reduce<<<G.n[0] + G.n[1] + G.n[2], 256, 0, s>>>(ppartials, G, B, out + 4);
+    return cudaGetLastError();
 }
 
 // lattice_measurement_wilson (wilson_loop.cl:55-454): per site and i in
@@ -761,21 +769,119 @@ __global__ void __launch_bounds__(128) k_wilson(Field<Real> U, Geom G, int R, in
     grid_sum<1, 128>(v, partials, ticket, out);
 }
 
+// The same loop with the lines shared: a block holds whole time columns (N4
+// <= 128 threads each) of one spatial direction i; thread (column, t) builds
+// the spatial line S(t) = L_i^R(x, t) once and leaves it in shared memory, and
+// the loop is Re Tr((L_t S(t+T)) (S(t) L_t')^+) with the time lines L_t =
+// L_t^T(x), L_t' = L_t^T(x+R i): (R-1) + 2 (T-1) + 2 products per (x, i, t)
+// against 2 (R-1) + (T-1) + 3 and (T-1)/3 of k_wilson, and half the link
+// loads and row-3 rebuilds.  Bound by the FP64 pipe.
+template <int NC, typename Real, bool TW>
+__global__ void __launch_bounds__(128) k_wilson_line(Field<Real> U, Geom G, int R, int T, int cols,
+                                                      const double *params, int twist, double *partials,
+                                                      unsigned *ticket, double *out)
+{
+    if (!TW) twist = 0;
+    __shared__ double S[18][128];
+    const int nt = G.n[3], tid = threadIdx.x;
+    const uint32_t Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
+    const int i = (int)(blockIdx.x % 3);                         // a group's three directions share its time links in L2
+    const int col = tid % cols, t = tid / cols;                  // neighbouring columns in neighbouring lanes
+    const uint32_t xs = blockIdx.x / 3 * cols + col;
+    const bool on = t < nt && xs < Vs;
+    double v[1] = { 0 };
+    Crd c = { 0, 0, 0, 0 };
+    M3<double> s;
+    if (on) {
+        c.y = (int)(xs % (uint32_t)G.n[1]);
+        const uint32_t r = xs / (uint32_t)G.n[1];
+        c.z = (int)(r % (uint32_t)G.n[2]);
+        c.x = (int)(r / (uint32_t)G.n[2]);
+        c.t = t;
+        s = load_d<NC, Real>(U, G, c, i, params, twist);
+        Crd a = c;
+#pragma unroll 1
+        for (int k = 1; k < R; k++) {
+            a = step_plus(G, a, i);
+            s = mulf(s, load_d<NC, Real>(U, G, a, i, params, twist));
+        }
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            S[2 * k][tid] = s.m[k / 3][k % 3].re;
+            S[2 * k + 1][tid] = s.m[k / 3][k % 3].im;
+        }
+        c = step_plus(G, a, i);                                  // x + R i
+    }
+    __syncthreads();
+    if (on) {
+        M3<double> l = load_d<NC, Real>(U, G, c, 3, params, twist);
+        Crd a = c;
+#pragma unroll 1
+        for (int k = 1; k < T; k++) { a = step_plus(G, a, 3); l = mulf(l, load_d<NC, Real>(U, G, a, 3, params, twist)); }
+        const M3<double> y = mulf(s, l);                         // S(t) L_t'
+        a.x = (int)(xs / (uint32_t)G.n[1] / (uint32_t)G.n[2]);
+        a.y = (int)(xs % (uint32_t)G.n[1]);
+        a.z = (int)(xs / (uint32_t)G.n[1] % (uint32_t)G.n[2]);
+        a.t = t;
+        l = load_d<NC, Real>(U, G, a, 3, params, twist);
+#pragma unroll 1
+        for (int k = 1; k < T; k++) { a = step_plus(G, a, 3); l = mulf(l, load_d<NC, Real>(U, G, a, 3, params, twist)); }
+        const int o = (t + T) % nt * cols + col;
+#pragma unroll
+        for (int k = 0; k < 9; k++) s.m[k / 3][k % 3] = { S[2 * k][o], S[2 * k + 1][o] };
+        double tr = 0;
+#pragma unroll
+        for (int p = 0; p < 3; p++)
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const CX<double> e = dot3(&l.m[p][0], 1, &s.m[0][q], 3);         // (L_t S(t+T))_pq
+                tr = FMA(e.re, y.m[p][q].re, tr);
+                tr = FMA(e.im, y.m[p][q].im, tr);
+            }
+        v[0] = tr;
+    }
+    grid_sum<1, 128>(v, partials, ticket, out);
+}
+
+// Columns per block, while they fill 3/4 of its threads; 0: k_wilson.  The
+// shared lines must save a third of the products: at 32^4 the 7 x 2 loop takes
+// 498 / 579 us against 655 / 661 (FP32 / FP64 links), the 2 x 2 loop 325 / 369
+// against 322 / 318, the 1 x 1 loop 211 / 239 against 196 / 193 (three times
+// the blocks, and a barrier between the lines and the loop).
+static int wilson_line_cols(const Geom &G, int R, int T)
+{
+    const int cols = G.n[3] <= 128 ? 128 / G.n[3] : 0;
+    const int line = 3 * ((R - 1) + 2 * (T - 1) + 2), site = 3 * (2 * (R - 1) + (T - 1) + 3) + (T - 1);
+    return cols * G.n[3] >= 96 && 3 * line < 2 * site ? cols : 0;
+}
+
+template <int NC, typename Real>
+static cudaError_t wilson_kernel(const Field<Real> &U, const Geom &G, int R, int T, const double *params, int twist,
+                                 double *partials, unsigned *ticket, double *out, cudaStream_t s)
+{
+    const uint32_t Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
+    const int cols = wilson_line_cols(G, R, T);
+    // at most 3 (V / 96 + 1) blocks: within the partials of a context
+    const uint32_t nb = cols ? 3 * ((Vs + cols - 1) / cols) : (G.V + 127) / 128;
+    unsigned *tk = fused_ticket(nb, ticket);
+    if (cols && twist) k_wilson_line<NC, Real, true><<<nb, 128, 0, s>>>(U, G, R, T, cols, params, twist, partials, tk, out);
+    else if (cols) k_wilson_line<NC, Real, false><<<nb, 128, 0, s>>>(U, G, R, T, cols, params, twist, partials, tk, out);
+    else if (twist) k_wilson<NC, Real, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out);
+    else k_wilson<NC, Real, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out);
+    return finish_sum(nb, 1, partials, out, s);
+}
+
 cudaError_t launch_wilson(const Geom &G, const void *links, int group, int prec, int R, int T, const double *params,
                           int twist, double *partials, unsigned *ticket, double *out, cudaStream_t s)
 {
-    uint32_t nb = (G.V + 127) / 128;
-    unsigned *tk = fused_ticket(nb, ticket);
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        if (group == 3) (twist ? k_wilson<3, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<3, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
-        else (twist ? k_wilson<2, double, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<2, double, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
-    } else {
-        Field<float> U{ (float4 *)links, G.pstride };
-        if (group == 3) (twist ? k_wilson<3, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<3, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
-        else (twist ? k_wilson<2, float, true><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out) : k_wilson<2, float, false><<<nb, 128, 0, s>>>(U, G, R, T, params, twist, partials, tk, out));
+        return group == 3 ? wilson_kernel<3, double>(U, G, R, T, params, twist, partials, ticket, out, s)
+                          : wilson_kernel<2, double>(U, G, R, T, params, twist, partials, ticket, out, s);
     }
-    return finish_sum(nb, 1, partials, out, s);
+    Field<float> U{ (float4 *)links, G.pstride };
+    return group == 3 ? wilson_kernel<3, float>(U, G, R, T, params, twist, partials, ticket, out, s)
+                      : wilson_kernel<2, float>(U, G, R, T, params, twist, partials, ticket, out, s);
 }
 
 // All planar Wilson loops R x T, R <= Rmax, T <= Tmax (<= 16), in one
