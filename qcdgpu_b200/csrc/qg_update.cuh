@@ -637,19 +637,23 @@ cudaError_t launch_after(void (*kern)(Field<Real>, Geom, PhaseArgs), unsigned nb
 // Launches k_phase_split with SP warps for 32 links; false where that is not
 // the faster form.  A block's registers stay taken while its first warp alone
 // updates the links, so the split pays while all blocks are resident with
-// room to spare: for SP = 6 up to 3/4 (SU(2): 3/5) of the resident blocks, for
-// SP = 3 up to 3/4 (with RANLUX batches, whose generator wants the SMs too,
-// 1/2).  Measured in the sweep graph, us a phase, heatbath / overrelaxation:
-//   SU(3) FP32  8^4   9.7 / 5.1 -> 6.6 / 2.7    16^3 x 8  10.3 / 5.1 -> 8.4 / 4.4
-//   SU(3) FP64  8^4  11.5 / 6.2 -> 7.0 / 3.6    16^3 x 8  12.1 / 6.5 -> 9.8 / 6.6
-//   SU(2) FP32  8^4   4.9 / 2.7 -> 2.6 / 1.5    16^4       5.5 / 3.1 -> 4.5 / 2.9
-//   SU(2) FP64  8^4   5.9 / 3.5 -> 2.7 / 1.7    16^3 x 8   6.2 / 3.6 -> 4.1 / 2.9
-// and beyond them, unsplit against SP = 3: SU(3) FP32 16^4 11.1 / 5.5 against
-// 13.1 / 6.2, FP64 14.3 / 8.4 against 16.9 / 11.2.  The early launch hides
-// the Philox heatbath's random numbers (SU(2) 8^4: 4.1 -> 2.6 us); without
-// them it only pays up to half a block per SM (the next phase's blocks
-// crowd where the first slots come free: SU(3) FP32 12^3 x 8
-// overrelaxation 3.2 us without, 4.2 with it, 4^4 2.65 / 2.31).
+// room to spare: SU(3) and the SU(2) heatbath with SP = 6 up to 3/4 (SU(2): 3/5)
+// of the resident blocks, then with SP = 3 up to 3/4 (FP32 overrelaxation and
+// RANLUX batches, whose generator wants the SMs too: 1/2; not the SU(2) FP64
+// heatbath); the SU(2) overrelaxation, little more than its loads, up to 128
+// blocks (FP64: 512).  Measured in the sweep graph, us a phase, heatbath /
+// overrelaxation, one thread per link -> split:
+//   SU(3) FP32  8^4   9.4 / 4.8 -> 6.6 / 2.7    16^3 x 8   9.7 / 4.9 -> 8.4 / 4.4
+//   SU(3) FP64  8^4  11.5 / 6.2 -> 7.0 / 3.6    16^3 x 8  11.9 / 6.4 -> 9.8 / 6.6
+//   SU(2) FP32  8^4   4.9 / 2.4 -> 2.6 / 1.5    16^4       5.1       -> 4.5
+//   SU(2) FP64  8^4   4.9 / 2.7 -> 2.7 / 1.7    16^3 x 8   5.2 / 2.9 -> 4.1 / 2.8
+// and beyond the limits: SU(3) FP32 16^4 10.9 / 5.3 against 13.1 / 6.2 with
+// SP = 3, FP64 14.3 / 8.4 against 16.9 / 11.2; SU(2) FP32 16^3 x 8
+// overrelaxation 1.9 against 2.6 with SP = 6.  The early launch hides the
+// Philox heatbath's random numbers (SU(2) 8^4: 4.1 -> 2.6 us); without them it
+// only pays up to half a block per SM (the next phase's blocks crowd where
+// the first slots come free: SU(3) FP32 12^3 x 8 overrelaxation 3.2 us
+// without, 4.2 with it, 4^4 2.65 / 2.31).
 template <int NC, typename Real, int PM, bool OR, int MU, int SP>
 bool try_split(const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStream_t s, cudaError_t &e)
 {
@@ -663,8 +667,12 @@ bool try_split(const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStre
         return n;
     }();
     const unsigned nb = (a.t_end - a.t_begin + 31) / 32, resident = 148u * per_sm;
-    const unsigned limit = SP == 6 ? (NC == 3 ? resident * 3 / 4 : resident * 3 / 5)
-                                   : (!OR && PM == 0 ? resident / 2 : resident * 3 / 4);
+    constexpr bool kF32 = sizeof(Real) == 4;
+    unsigned limit;
+    if (NC == 2 && OR) limit = SP == 6 ? (kF32 ? 128 : 512) : 0;
+    else if (SP == 6) limit = NC == 3 ? resident * 3 / 4 : resident * 3 / 5;
+    else if (NC == 2 && !kF32) limit = 0;
+    else limit = (OR && kF32) || (!OR && PM == 0) ? resident / 2 : resident * 3 / 4;
     if (nb > limit) return false;
     const bool early = a.after_phase && ((!OR && PM == 1) || nb <= 74);
     e = launch_after(k_phase_split<NC, Real, PM, OR, MU, SP>, nb, 32 * SP, early, U, G, a, s);
@@ -727,10 +735,18 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
     // (32^4: SU(3) FP32 overrelaxation 52.2 -> 50.1 us in shape 1, 52.6 ->
     // 51.8 in shape 3, SU(2) FP32 11.1 -> 10.6; 24^4 2-4 %); with fewer they
     // crowd on the SMs whose blocks end first (16^4 5.5 -> 9.6 us)
-    const bool early = a.after_phase && nb >= 1024;
+    const bool early = a.after_phase && a.t_end - a.t_begin >= 1024 * kPhaseBlock;
     // shape 0 of few links: six or three warps for 32 links (k_phase_split)
     cudaError_t e;
     if (a.variant == 0 && !a.twist && pm != 2 && launch_phase_split<Real>(U, G, group, a, s, e)) return e;
+    // shape 0 otherwise: the compiler's registers, or the form held to five
+    // blocks per SM (shape 1) where that is the faster: SU(3) FP32 (us a phase,
+    // heatbath / overrelaxation: 20^4 19.2 / 10.2 -> 17.2 / 9.6, 24^4 31.4 / 16.5
+    // -> 29.8 / 15.9, 32^4 92.8 / 54.9 -> 88.4 / 51.2) and SU(2) up to 100 000
+    // links (FP32 16^4 5.6 / 3.1 -> 5.1 / 2.4, FP64 6.9 / 4.0 -> 5.7 / 3.4; at 32^4
+    // the FP64 heatbath 39.6 against 44.4); SU(3) FP64 spills (16^4 14.4 / 8.4
+    // against 17.8 / 11.0)
+    const bool tight = group == 3 ? kStage : a.t_end - a.t_begin <= 100000;
     // twisted boundaries: shape 0's form with the twist tests compiled in
     // (any shape computes the same sequence); the others are compiled
     // without them
@@ -742,6 +758,7 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
         else if (a.variant == 2) QG_LAUNCH2(NC, PM, OR, MU, 6, false);              \
         else if (a.variant == 3) QG_LAUNCH2(NC, PM, OR, MU, 0, NC == 3 && kStage);  \
         else if (a.variant >= 4) QG_LAUNCH2(NC, PM, OR, MU, 5, NC == 3 && kStage);  \
+        else if (tight) QG_LAUNCH2(NC, PM, OR, MU, 5, false);                       \
         else QG_LAUNCH2(NC, PM, OR, MU, 0, false);                                  \
     } while (0)
 #define QG_LAUNCH(NC, PM, OR)                                     \
