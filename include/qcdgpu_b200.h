@@ -162,8 +162,10 @@ int qg_sweep_phase_times(qg_ctx *ctx, int nsweeps, double *ms_heatbath, double *
 /* Autotuner (new): times each launch shape of the heatbath and the
  * overrelaxation phase kernels on this context's lattice (`reps` launches
  * each; the field is restored and no PRN counter moves) and keeps the
- * fastest for later phases and sweeps.  Shapes: 0 = links loaded straight
- * into registers, compiler's register count; 1, 2 = the same held to 5 / 6
+ * fastest for later phases and sweeps.  Shapes: 0 (the default) = chosen by
+ * the number of links: a link's staple terms over several warps while the
+ * links fill less than the GPU, else one thread per link, its links loaded
+ * straight into registers; 1, 2 = one thread per link held to 5 / 6
  * resident blocks per SM; 3, 4 = staple links streamed through shared
  * memory two staple terms ahead (SU(3) FP32; other cases run shape 0 / 1);
  * 5 = overrelaxation two links per thread with packed FP32 (FFMA2)
@@ -239,11 +241,12 @@ int qg_measure_enqueue(qg_ctx *ctx, int what, uint64_t *ticket);
 int qg_measure_fetch(qg_ctx *ctx, uint64_t ticket, double *out);
 /* same, generalised Wilson loop of extent R x T (config keys WILSONR/T)   */
 int qg_measure_wilson(qg_ctx *ctx, int R, int T, double *out);
-/* all planar Wilson loops R x T for R <= Rmax, T <= Tmax (both <= 16): in
- * one launch, out[(R-1)*Tmax + (T-1)] = the raw sum qg_measure_wilson
+/* all planar Wilson loops R x T for R <= Rmax, T <= Tmax (both <= 16) in
+ * one call, out[(R-1)*Tmax + (T-1)] = the raw sum qg_measure_wilson
  * gives (new; the reference measures one R x T per run).  fp64_products:
  * 1 = matrix products in FP64 as qg_measure_wilson; 0 = in FP32 on FP32
- * links (traces summed in FP64; about 4x faster, relative error ~1e-6)  */
+ * links where that is faster (few loops; traces summed in FP64, relative
+ * error ~1e-6; many loops are taken with FP64 products either way)        */
 int qg_measure_wilson_all(qg_ctx *ctx, int Rmax, int Tmax, int fp64_products, double *out);
 
 /* F_munu: the projections -i Tr(P T_a) of every plaquette P of three planes

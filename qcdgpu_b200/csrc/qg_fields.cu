@@ -374,12 +374,13 @@ cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint
     if (st.bytes < want && !st.reduced) {
         ref_stage_free(st);
         size_t n = want;
-        cudaError_t e = cudaMalloc(&st.p, n);
+        // from the stream's pool: a first table costs no device-wide allocation
+        cudaError_t e = cudaMallocAsync(&st.p, n, s);
         while (e == cudaErrorMemoryAllocation && n / 2 >= kRefStageMin) {
             cudaGetLastError();                          // not left pending for the next launch check
             n /= 2;
             st.reduced = true;
-            e = cudaMalloc(&st.p, n);
+            e = cudaMallocAsync(&st.p, n, s);
         }
         if (e != cudaSuccess) {
             st = RefStage{};

@@ -759,7 +759,7 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
         else if (a.variant == 3) QG_LAUNCH2(NC, PM, OR, MU, 0, NC == 3 && kStage);  \
         else if (a.variant >= 4) QG_LAUNCH2(NC, PM, OR, MU, 5, NC == 3 && kStage);  \
         else if (tight) QG_LAUNCH2(NC, PM, OR, MU, 5, false);                       \
-        else QG_LAUNCH2(NC, PM, OR, MU, 0, false);                                  \
+        else QG_LAUNCH2(NC, PM, OR, MU, NC == 3 && kStage ? 5 : 0, false);          \
     } while (0)
 #define QG_LAUNCH(NC, PM, OR)                                     \
     do {                                                          \
