@@ -18,6 +18,12 @@ struct Twist {
     int xlast;
 };
 
+// Staple links by the read-only path (ld.global.nc).  It is defined only for
+// data that nothing writes while the kernel is resident, so a kernel that
+// takes it starts after the phase before has ended: k_phase is never a
+// programmatic dependent (k_phase_split, which is, reads with ordinary
+// loads).  Ordinary loads and the early launch are not the faster pair: 32^4
+// SU(3) FP64 heatbath 159 -> 173 us, FP32 overrelaxation in shape 1 50.5 -> 55.4.
 template <typename Real>
 __device__ __forceinline__ G3<Real> load3t(const Field<Real> &U, int dir, uint32_t e, int xc, const Twist<Real> &tw)
 {
@@ -343,9 +349,7 @@ __device__ __forceinline__ void phase_site(const Field<Real> &U, const Geom &G, 
 template <int NC, typename Real, int PMODE, bool OR, int mu, int MINB, bool STAGED, bool TW>
 __global__ void __launch_bounds__(kPhaseBlock, MINB) k_phase(Field<Real> U, Geom G, PhaseArgs A)
 {
-    grid_dependents_may_start();
     const uint32_t t = A.t_begin + blockIdx.x * blockDim.x + threadIdx.x;
-    grid_dependency_wait();
     if (t >= A.t_end) return;
     if constexpr (STAGED) {
         __shared__ __align__(16) StageBuf sb;
@@ -731,11 +735,6 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
             return cudaGetLastError();
         }
     }
-    // many blocks: the next phase's first blocks start in this one's last wave
-    // (32^4: SU(3) FP32 overrelaxation 52.2 -> 50.1 us in shape 1, 52.6 ->
-    // 51.8 in shape 3, SU(2) FP32 11.1 -> 10.6; 24^4 2-4 %); with fewer they
-    // crowd on the SMs whose blocks end first (16^4 5.5 -> 9.6 us)
-    const bool early = a.after_phase && a.t_end - a.t_begin >= 1024 * kPhaseBlock;
     // shape 0 of few links: six or three warps for 32 links (k_phase_split)
     cudaError_t e;
     if (a.variant == 0 && !a.twist && pm != 2 && launch_phase_split<Real>(U, G, group, a, s, e)) return e;
@@ -750,10 +749,10 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
     // twisted boundaries: shape 0's form with the twist tests compiled in
     // (any shape computes the same sequence); the others are compiled
     // without them
-#define QG_LAUNCH2(NC, PM, OR, MU, MB, ST) return launch_after(k_phase<NC, Real, PM, OR, MU, MB, ST, false>, nb, bs, early, U, G, a, s)
+#define QG_LAUNCH2(NC, PM, OR, MU, MB, ST) k_phase<NC, Real, PM, OR, MU, MB, ST, false><<<nb, bs, 0, s>>>(U, G, a)
 #define QG_LAUNCH1(NC, PM, OR, MU)                                                  \
     do {                                                                            \
-        if (a.twist) return launch_after(k_phase<NC, Real, PM, OR, MU, 0, false, true>, nb, bs, early, U, G, a, s); \
+        if (a.twist) k_phase<NC, Real, PM, OR, MU, 0, false, true><<<nb, bs, 0, s>>>(U, G, a); \
         else if (a.variant == 1) QG_LAUNCH2(NC, PM, OR, MU, 5, false);              \
         else if (a.variant == 2) QG_LAUNCH2(NC, PM, OR, MU, 6, false);              \
         else if (a.variant == 3) QG_LAUNCH2(NC, PM, OR, MU, 0, NC == 3 && kStage);  \
@@ -784,6 +783,7 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
 #undef QG_LAUNCH
 #undef QG_LAUNCH1
 #undef QG_LAUNCH2
+    return cudaGetLastError();
 }
 
 }  // namespace qg

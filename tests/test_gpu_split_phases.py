@@ -2,7 +2,8 @@
 warps, shape 0) against the one-thread-per-link kernels (shape 1), link by
 link: blocks that are not full, the sizes on both sides of each limit, long
 reject chains (random quads beyond the precomputed ones), several hits, the
-RANLUX stream, and the graph's early launches against single phases."""
+RANLUX stream, and the graph's early launches against single phases (and
+that large lattices, whose phases follow one another, equal them too)."""
 import numpy as np
 import pytest
 
@@ -58,3 +59,51 @@ def test_graph_sweeps_equal_single_phases(prng):
     L.reunitarize()
     assert np.array_equal(L.download(), chain(0, 2, **kw))
     L.close()
+
+
+def single_phases(L, n_or, ranlux):
+    """two sweeps by single phase launches, none of them in a graph"""
+    for _ in range(2):
+        for kind in [Q.HEATBATH] + [Q.OVERRELAX] * n_or:
+            for p in (1, 0):
+                for d in range(4):
+                    if ranlux and kind == Q.HEATBATH:
+                        L.produce()
+                    L.phase(p, d, kind)
+    L.reunitarize()
+
+
+@pytest.mark.parametrize("group,precision", [(3, 0), (3, 1), (2, 0), (2, 1)])
+@pytest.mark.parametrize("size", [(24, 24, 24, 6), (20, 20, 20, 20), (24, 24, 24, 20)])
+@pytest.mark.parametrize("mode", ["philox", "twisted", "ranlux"])
+def test_every_shape_in_the_graph_equals_single_phases(group, precision, size, mode):
+    """a phase reads links that the phase before wrote: whatever a graph lets
+    overlap, the chain is that of launches one after another, for every shape
+    and on both sides of 2^17 links a phase"""
+    kw = dict(group=group, precision=precision, size=size, beta=5.9 if group == 3 else 2.3, n_or=1, nhit=4,
+              prng=Q.PRNG_RANLUX if mode == "ranlux" else Q.PRNG_PHILOX, prng_instances=16384, start=Q.START_HOT,
+              randseries=7, reunit_every=2)
+    if mode == "twisted":
+        kw.update(phi=0.4, omega=0.9)
+    L = Q.Lattice(Q.default_config(**kw))
+
+    def begin():
+        L.seed()
+        L.init(Q.START_HOT)
+
+    begin()
+    start = L.download()
+    L.set_shapes(1, 1)
+    single_phases(L, 1, mode == "ranlux")
+    want = L.download()
+    assert not np.array_equal(want, start)
+    L.close()
+    for look in ([True, False] if mode == "ranlux" else [True]):
+        for shape in [0] if mode == "twisted" else [0, 3] if mode == "ranlux" else range(Q.TUNE_SHAPES):
+            L = Q.Lattice(Q.default_config(**kw))
+            L.set_prng_lookahead(look)
+            begin()
+            L.set_shapes(shape, shape)
+            L.sweep(2)
+            assert np.array_equal(L.download(), want), (look, shape)
+            L.close()
