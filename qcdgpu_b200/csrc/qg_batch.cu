@@ -189,7 +189,7 @@ __device__ __forceinline__ void tiles_of_phase(const EnsDesc *ens, const uint32_
         A.t_end = G.half;
         A.t_prn = 0;
         A.after_phase = 0;
-        Field<Real> U;
+        Field<Real, false> U;                         // the launch writes links that its later directions read
         U.p = reinterpret_cast<typename V4<Real>::T *>(d.links);
         U.pstride = G.pstride;
         phase_site<NC, Real, 1, OR, mu, STAGED>(U, G, A, t, sb);

@@ -133,12 +133,16 @@ __device__ __forceinline__ void st4(double4 *p, const R4<double> &v)
     q[1] = make_double2(v.z, v.w);
 }
 
-template <typename Real>
+// RO: ldg3 and ldg2 take the read-only path (ld.global.nc), which is defined
+// only for links that nothing writes while the kernel is resident; false for
+// a kernel that runs several phases
+template <typename Real, bool RO = true>
 struct Field {
     typename V4<Real>::T *p;
     uint32_t pstride;
     __device__ __forceinline__ G3<Real> ldg3(int dir, uint32_t e) const
     {
+        if constexpr (!RO) return ld3(dir, e);
         G3<Real> m;
         m.uv1 = ldg4(p + (size_t)dir * pstride + e);
         m.uv2 = ldg4(p + (size_t)(dir + 4) * pstride + e);
@@ -159,7 +163,11 @@ struct Field {
         st4(p + (size_t)(dir + 4) * pstride + e, m.uv2);
         st4(p + (size_t)(dir + 8) * pstride + e, m.uv3);
     }
-    __device__ __forceinline__ R4<Real> ldg2(int dir, uint32_t e) const { return ldg4(p + (size_t)dir * pstride + e); }
+    __device__ __forceinline__ R4<Real> ldg2(int dir, uint32_t e) const
+    {
+        if constexpr (!RO) return ld2(dir, e);
+        return ldg4(p + (size_t)dir * pstride + e);
+    }
     __device__ __forceinline__ R4<Real> ld2(int dir, uint32_t e) const { return ld4(p + (size_t)dir * pstride + e); }
     __device__ __forceinline__ void st2(int dir, uint32_t e, const R4<Real> &m) const { st4(p + (size_t)dir * pstride + e, m); }
 };

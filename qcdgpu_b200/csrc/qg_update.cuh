@@ -18,21 +18,22 @@ struct Twist {
     int xlast;
 };
 
-// Staple links by the read-only path (ld.global.nc).  It is defined only for
-// data that nothing writes while the kernel is resident, so a kernel that
-// takes it starts after the phase before has ended: k_phase is never a
-// programmatic dependent (k_phase_split, which is, reads with ordinary
+// Staple links by the read-only path (ld.global.nc) where the field allows it
+// (RO).  It is defined only for data that nothing writes while the kernel is
+// resident, so a kernel that takes it runs one phase and starts after the
+// phase before has ended: k_phase is never a programmatic dependent
+// (k_phase_split, which is, and the persistent half-sweep read with ordinary
 // loads).  Ordinary loads and the early launch are not the faster pair: 32^4
 // SU(3) FP64 heatbath 159 -> 173 us, FP32 overrelaxation in shape 1 50.5 -> 55.4.
-template <typename Real>
-__device__ __forceinline__ G3<Real> load3t(const Field<Real> &U, int dir, uint32_t e, int xc, const Twist<Real> &tw)
+template <typename Real, bool RO>
+__device__ __forceinline__ G3<Real> load3t(const Field<Real, RO> &U, int dir, uint32_t e, int xc, const Twist<Real> &tw)
 {
     G3<Real> m = U.ldg3(dir, e);
     if (tw.on && dir == 1 && xc == tw.xlast) m = twist3(m, tw.phi, tw.omega);
     return m;
 }
-template <typename Real>
-__device__ __forceinline__ R4<Real> load2t(const Field<Real> &U, int dir, uint32_t e, int xc, const Twist<Real> &tw)
+template <typename Real, bool RO>
+__device__ __forceinline__ R4<Real> load2t(const Field<Real, RO> &U, int dir, uint32_t e, int xc, const Twist<Real> &tw)
 {
     R4<Real> m = U.ldg2(dir, e);
     if (tw.on && dir == 1 && xc == tw.xlast) {
@@ -82,8 +83,8 @@ __device__ __forceinline__ Nbr neighbours(const Geom &G, const Crd &c)
 // plane nu the forward term U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+ and the
 // backward term U_nu(x-nu+mu)^+ U_mu(x-nu)^+ U_nu(x-nu), summed as
 // st = f0 + b0; st = b_i + (st + f_i)
-template <int mu, typename Real>
-__device__ __forceinline__ M3<Real> staple3(const Field<Real> &U, const Geom &G, uint32_t t, const Nbr &n, int p,
+template <int mu, typename Real, bool RO>
+__device__ __forceinline__ M3<Real> staple3(const Field<Real, RO> &U, const Geom &G, uint32_t t, const Nbr &n, int p,
                                            const Twist<Real> &tw)
 {
     const uint32_t own = (uint32_t)p * G.cb + t, opp = (uint32_t)(p ^ 1) * G.cb + t;
@@ -108,8 +109,8 @@ __device__ __forceinline__ M3<Real> staple3(const Field<Real> &U, const Geom &G,
     return st;
 }
 
-template <int mu, typename Real>
-__device__ __forceinline__ S2<Real> staple2(const Field<Real> &U, const Geom &G, uint32_t t, const Nbr &n, int p,
+template <int mu, typename Real, bool RO>
+__device__ __forceinline__ S2<Real> staple2(const Field<Real, RO> &U, const Geom &G, uint32_t t, const Nbr &n, int p,
                                            const Twist<Real> &tw)
 {
     const uint32_t own = (uint32_t)p * G.cb + t, opp = (uint32_t)(p ^ 1) * G.cb + t;
@@ -301,8 +302,8 @@ __device__ __forceinline__ R4<Real> su2_update(const S2<Real> &st, const R4<Real
 // every twist test folds away at compile time (4 % of the phase's time)
 // sb: the block's staging buffer (STAGED; declared by the kernel, so that a
 // kernel running several directions holds one)
-template <int NC, typename Real, int PMODE, bool OR, int mu, bool STAGED, bool TW = false>
-__device__ __forceinline__ void phase_site(const Field<Real> &U, const Geom &G, const PhaseArgs &A, uint32_t t,
+template <int NC, typename Real, int PMODE, bool OR, int mu, bool STAGED, bool TW = false, bool RO = true>
+__device__ __forceinline__ void phase_site(const Field<Real, RO> &U, const Geom &G, const PhaseArgs &A, uint32_t t,
                                            StageBuf *sb)
 {
     const int p = A.parity;
@@ -323,7 +324,7 @@ __device__ __forceinline__ void phase_site(const Field<Real> &U, const Geom &G, 
         G3<Real> m0;
         M3<Real> st;
         if constexpr (STAGED) {
-            st = staple3_staged<mu>(U, G, t, nb, p, tw, *sb, m0);
+            st = staple3_staged<mu>(Field<Real>{ U.p, U.pstride }, G, t, nb, p, tw, *sb, m0);
         } else {
             m0 = U.ld3(mu, e0);
             st = staple3<mu>(U, G, t, nb, p, tw);
