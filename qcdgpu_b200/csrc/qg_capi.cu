@@ -1404,7 +1404,7 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
     // are latency (4^4, 4 x 4: 53 us either way; 8^4, 5 x 5: 65 against 89 us
     // whatever the products).  The column kernel also
     // where a line is larger than the scratch, the scratch is not free, or a
-    // time line is too far from SU(N) to be inverted.  One buffer: results
+    // time line is too far from unitary to be inverted.  One buffer: results
     // (257), slots, scratch
     const bool gauge = nl >= (c->G.V <= 4096 ? 25 : (f.precision || fp64_products) ? 16 : 32);
     const size_t scratch = gauge ? wilson_lines_scratch(c->G, f.group, Tmax) : 0;

@@ -93,7 +93,7 @@ cudaError_t launch_wilson_all(const Geom &G, const void *links, int group, int p
 // wilson_lines_scratch bytes (0: a line does not fit, take
 // launch_wilson_all), slots of wilson_lines_slots doubles; out holds
 // Rmax Tmax sums and then a flag, non-zero when a time line is too far from
-// SU(N) for its inverse to be taken (the sums are then not to be used)
+// unitary for its inverse to be taken (the sums are then not to be used)
 size_t wilson_lines_scratch(const Geom &G, int group, int Tmax);
 size_t wilson_lines_slots(int Rmax, int Tmax);
 cudaError_t launch_wilson_lines(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,

@@ -72,6 +72,28 @@ def test_links_off_su3(twist):
     L.close()
 
 
+@pytest.mark.parametrize("size,loops", [((4, 4, 4, 64), (4, 8)), ((4, 4, 4, 150), (4, 10)), ((8, 6, 8, 16), (4, 6))])
+def test_time_lines_near_singular_with_unit_determinant(size, loops):
+    """row 1 of every link times s, row 2 over s, s = e^(+-0.4): determinants stay 1 while a time line grows
+    singular to rounding (its condition to 1e8 at N4 = 64), so no loop may be taken through its inverse"""
+    L = lattice(3, size, 1)
+    t = L.download().reshape(12, -1, 4)
+    g = np.exp(0.4 * np.random.default_rng(5).choice([-1.0, 1.0], size=(4,) + t.shape[1:2]))
+    t[0:8, :, :3] *= np.tile(g, (2, 1))[:, :, None]      # row 1: x, y, z of planes 0-3 (real), 4-7 (imaginary)
+    t[0:8, :, 3] /= np.tile(g, (2, 1))                   # row 2: w there, and planes 8-11
+    t[8:12] /= g[:, :, None]
+    L.upload(t.ravel())
+    R, T = loops
+    W = L.wilson_all(R, T)
+    V = float(L.info().sites)
+    for r, u in [(1, 1), (1, T), (2, 2), (R, T)]:
+        n = 2 * (r + u)
+        # n factors of norm e^0.4, some 8 roundings a product, traces of size 3 of 3 V loops, twice (both sides)
+        tol = 2 * 3 * V * 3 * n * 8 * 1.2e-16 * np.exp(0.4 * n)
+        assert abs(W[r - 1, u - 1] - L.wilson_sum(r, u)) <= tol, (r, u, W[r - 1, u - 1], L.wilson_sum(r, u), tol)
+    L.close()
+
+
 def test_time_lines_without_an_inverse_take_the_general_path():
     """a field of zeros (a context that was never started) has sums 0"""
     L = Q.Lattice(Q.default_config(group=3, size=(6, 6, 6, 6), precision=0, prng=Q.PRNG_PHILOX))
