@@ -337,7 +337,7 @@ struct qg_batch {
     int shape_hb = 4, shape_or = 4;    // phase-kernel launch shapes (qg_batch_tune)
     bool persistent = false;           // one launch per half-sweep (qg_batch_set_persistent)
     bool plaq_fp32 = false;            // FP32-product plaquette (qg_batch_set_measure_products)
-    RefStage stage;                    // reference-layout table copies (lazy)
+    Scratch scratch;                   // reference-layout table copies (lazy)
     GridBarrier *d_bar = nullptr;
     unsigned *d_tiles = nullptr;       // the persistent half-sweep's tile counters, one per direction
 };
@@ -574,7 +574,7 @@ extern "C" int qg_batch_destroy(qg_batch *b)
     cudaFree(b->d_series);
     cudaFree(b->d_bar);
     cudaFree(b->d_tiles);
-    ref_stage_free(b->stage);
+    scratch_free(b->scratch);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return QG_OK;
@@ -868,7 +868,7 @@ extern "C" int qg_batch_links_download(qg_batch *b, int e, void *host)
     const qg_config &c = b->cfg;
     const uint32_t a = c.row_align > 0 ? (uint32_t)c.row_align : 64;
     const uint32_t rowsize = (G.V + a - 1) / a * a;
-    QB_CK(ref_stage_copy(G, (char *)b->links + b->offset[e], c.group, c.precision, rowsize, host, true, b->stage,
+    QB_CK(ref_table_copy(G, (char *)b->links + b->offset[e], c.group, c.precision, rowsize, host, true, b->scratch,
                          b->stream), "batch download");
     QB_CK(cudaStreamSynchronize(b->stream), "batch download");
     return QG_OK;

@@ -13,6 +13,9 @@
 
 using namespace qg;
 
+// Rmax Tmax <= 256 sums and a flag (qg_measure_wilson_all)
+constexpr int kLoopResults = 257;
+
 struct qg_ctx {
     qg_config cfg;
     Geom G;
@@ -26,7 +29,7 @@ struct qg_ctx {
     uint32_t *d_seeds = nullptr;
     double *partials = nullptr;
     size_t partials_n = 0;
-    double *d_results = nullptr;
+    double *d_results = nullptr;    // 64, then kLoopResults of the all-loops measurement
     double *h_results = nullptr;    // pinned; the observables' kernels write here
     unsigned *d_ticket = nullptr;   // their block counter (in d_results)
     uint64_t *d_phase = nullptr;
@@ -69,17 +72,13 @@ struct qg_ctx {
     bool slab = false;
     int slab_x0 = 0, slab_n1 = 0;
     unsigned long long *d_bad = nullptr;   // qg_field_check counter
-    RefStage stage;                 // reference-layout table copies (lazy)
+    Scratch scratch;                // link table copies and the all-loops measurement (lazy)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_phase[8] = {};
     // learned-proposal Metropolis (qg_net_*, qg_mh_*)
     uint16_t *d_netw = nullptr;     // BF16 weights the kernels read
     float *d_master = nullptr, *d_adam_m = nullptr, *d_adam_v = nullptr;
     float *d_grad = nullptr, *d_gpart = nullptr;    // QG_NET_PARAMS + 4 stats; per-block partials
-    double *d_wpart = nullptr;      // all-loops Wilson measurement, column kernel (lazy)
-    int wpart_rmax = 0;
-    double *d_wline = nullptr;      // the same: results, and slots and scratch of the time-line gauge (lazy)
-    size_t wline_bytes = 0;
     double *d_fpart = nullptr, *d_ppart = nullptr, *d_pout = nullptr;   // F_munu / profiles (lazy)
     double *d_sites = nullptr;      // per-site values of the one-pass measurements (lazy)
     unsigned long long *d_mh_acc = nullptr;
@@ -239,10 +238,9 @@ extern "C" int qg_destroy(qg_ctx *c)
     cudaFree(c->d_netw); cudaFree(c->d_master); cudaFree(c->d_adam_m); cudaFree(c->d_adam_v);
     cudaFree(c->d_grad); cudaFree(c->d_gpart); cudaFree(c->d_mh_acc); cudaFree(c->d_mh_jump);
     cudaFree(c->d_net_err); cudaFree(c->d_eps);
-    cudaFree(c->d_wpart); cudaFree(c->d_wline);
     cudaFree(c->d_fpart); cudaFree(c->d_ppart); cudaFree(c->d_pout); cudaFree(c->d_sites);
     cudaFree(c->d_bad);
-    ref_stage_free(c->stage);
+    scratch_free(c->scratch);
     if (c->h_results) cudaFreeHost(c->h_results);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_ring) cudaFreeHost(c->h_ring);
@@ -313,7 +311,7 @@ extern "C" int qg_create(const qg_config *cfg, qg_ctx **out)
         }
     }
     if ((e = cudaMalloc(&c->partials, c->partials_n * sizeof(double))) != cudaSuccess) return bad("cudaMalloc(partials)");
-    if ((e = cudaMalloc(&c->d_results, 64 * sizeof(double))) != cudaSuccess) return bad("cudaMalloc(results)");
+    if ((e = cudaMalloc(&c->d_results, (64 + kLoopResults) * sizeof(double))) != cudaSuccess) return bad("cudaMalloc(results)");
     c->d_ticket = reinterpret_cast<unsigned *>(c->d_results + 63);
     if ((e = cudaMemsetAsync(c->d_ticket, 0, sizeof(double), c->stream)) != cudaSuccess) return bad("cudaMemset(ticket)");
     if ((e = cudaMallocHost(&c->h_results, 64 * sizeof(double))) != cudaSuccess) return bad("cudaMallocHost");
@@ -1404,32 +1402,16 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
     // are latency (4^4, 4 x 4: 53 us either way; 8^4, 5 x 5: 65 against 89 us
     // whatever the products).  The column kernel also
     // where a line is larger than the scratch, the scratch is not free, or a
-    // time line is too far from unitary to be inverted.  One buffer: results
-    // (257), slots, scratch
+    // time line is too far from unitary to be inverted.
     const bool gauge = nl >= (c->G.V <= 4096 ? 25 : (f.precision || fp64_products) ? 16 : 32);
-    const size_t scratch = gauge ? wilson_lines_scratch(c->G, f.group, Tmax) : 0;
-    const size_t head = (257 + wilson_lines_slots(Rmax, Tmax) + 31) / 32 * 32 * sizeof(double);     // 256-byte aligned
-    const size_t want = scratch ? head + scratch : 257 * sizeof(double);
-    if (want > c->wline_bytes) {
-        cudaFree(c->d_wline);
-        c->d_wline = nullptr;
-        c->wline_bytes = 0;
-        cudaError_t e = cudaMalloc(&c->d_wline, want);
-        size_t got = want;
-        if (e == cudaErrorMemoryAllocation && scratch) {
-            cudaGetLastError();
-            got = 257 * sizeof(double);
-            e = cudaMalloc(&c->d_wline, got);
-        }
-        QG_CK(e, "wilson scratch");
-        c->wline_bytes = got;
-    }
-    double *d_wout = c->d_wline;
-    if (scratch && c->wline_bytes >= want) {
+    const size_t lines = gauge ? wilson_lines_scratch(c->G, f.group, Rmax, Tmax) : 0;
+    double *d_wout = c->d_results + 64;
+    cudaError_t e = lines ? scratch_reserve(c->scratch, lines, lines, c->stream) : cudaErrorMemoryAllocation;
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "wilson scratch");
+    if (e == cudaSuccess) {
         QG_CK(launch_wilson_lines(c->G, c->links, f.group, f.precision, Rmax, Tmax, c->d_params, tw,
-                                  c->d_wline + head / sizeof(double), scratch, c->d_wline + 257, d_wout, c->stream),
-              "wilson all");
-        double h[257];
+                                  (double *)c->scratch.p, lines, d_wout, c->stream), "wilson all");
+        double h[kLoopResults];
         QG_CK(cudaMemcpyAsync(h, d_wout, (size_t)(nl + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
               "wilson copy");
         QG_CK(cudaStreamSynchronize(c->stream), "wilson sync");
@@ -1438,16 +1420,10 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
             return QG_OK;
         }
     }
-    if (c->wpart_rmax < Rmax) {
-        cudaFree(c->d_wpart);
-        c->d_wpart = nullptr;
-        c->wpart_rmax = 0;
-        QG_CK(cudaMalloc(&c->d_wpart, wilson_all_partials(wilson_all_blocks(c->G), Rmax) * sizeof(double)),
-              "wilson scratch");
-        c->wpart_rmax = Rmax;
-    }
+    const size_t cols = wilson_all_partials(wilson_all_blocks(c->G), Rmax) * sizeof(double);
+    QG_CK(scratch_reserve(c->scratch, cols, cols, c->stream), "wilson scratch");
     QG_CK(launch_wilson_all(c->G, c->links, f.group, f.precision, Rmax, Tmax, fp64_products, c->d_params, tw,
-                            c->d_wpart, d_wout, c->stream), "wilson all");
+                            (double *)c->scratch.p, d_wout, c->stream), "wilson all");
     QG_CK(cudaMemcpyAsync(out, d_wout, (size_t)nl * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
           "wilson copy");
     QG_CK(cudaStreamSynchronize(c->stream), "wilson sync");
@@ -1593,8 +1569,8 @@ extern "C" int qg_links_upload(qg_ctx *c, const void *host, int layout)
 {
     if (!c || !host) return QG_ERR_ARG;
     if (layout != QG_LAYOUT_REFERENCE) return fail(c, QG_ERR_ARG, "unknown layout");
-    QG_CK(ref_stage_copy(c->G, c->links, c->cfg.group, c->cfg.precision, c->rowsize, const_cast<void *>(host), false,
-                         c->stage, c->stream), "links upload");
+    QG_CK(ref_table_copy(c->G, c->links, c->cfg.group, c->cfg.precision, c->rowsize, const_cast<void *>(host), false,
+                         c->scratch, c->stream), "links upload");
     QG_CK(cudaStreamSynchronize(c->stream), "upload sync");
     return QG_OK;
 }
@@ -1603,7 +1579,7 @@ extern "C" int qg_links_download(qg_ctx *c, void *host, int layout)
 {
     if (!c || !host) return QG_ERR_ARG;
     if (layout != QG_LAYOUT_REFERENCE) return fail(c, QG_ERR_ARG, "unknown layout");
-    QG_CK(ref_stage_copy(c->G, c->links, c->cfg.group, c->cfg.precision, c->rowsize, host, true, c->stage, c->stream),
+    QG_CK(ref_table_copy(c->G, c->links, c->cfg.group, c->cfg.precision, c->rowsize, host, true, c->scratch, c->stream),
           "links download");
     QG_CK(cudaStreamSynchronize(c->stream), "download sync");
     return QG_OK;

@@ -346,69 +346,65 @@ static cudaError_t launch_ref_piece(const Geom &G, void *links, void *ref, int p
     return cudaGetLastError();
 }
 
-// The reference-layout link table to or from host memory through a staging
-// buffer that the owner of the field keeps (at most kRefStageBytes; smaller
-// when the table is, or when that much is not free): whole planes, or
-// pieces of one plane, each converted and copied in stream order.  A buffer
+namespace {
+struct StreamMemory {
+    using Error = cudaError_t;
+    static constexpr Error kSuccess = cudaSuccess, kNoMemory = cudaErrorMemoryAllocation;
+    cudaStream_t s;
+    Error alloc(void **p, size_t n)
+    {
+        // from the stream's pool: a first buffer costs no device-wide allocation
+        const Error e = cudaMallocAsync(p, n, s);
+        if (e == kNoMemory) cudaGetLastError();          // not left pending for the next launch check
+        return e;
+    }
+    void free(void *p) { if (p) cudaFreeAsync(p, s); }
+    void sync() { cudaStreamSynchronize(s); }
+};
+}  // namespace
+
+cudaError_t scratch_reserve(Scratch &st, size_t want, size_t least, cudaStream_t s)
+{
+    StreamMemory m{ s };
+    return scratch_reserve(m, st, want, least);
+}
+
+void scratch_free(Scratch &st)
+{
+    cudaFree(st.p);
+    st = Scratch{};
+}
+
+// The reference-layout link table to or from host memory through the scratch
+// that the owner of the field keeps (at most kScratchBytes; smaller when the
+// table is, or when that much is not free).  A buffer
 // of the whole table from the stream-ordered pool was unmapped at every
 // synchronisation and mapped again by the next call (a 32^4 FP32 table of
 // 201 MB in, checked, reunitarised, measured and out: 14.6 ms so, 7.8 ms
 // with the kept buffer; a 98 KB one at 4^4 in a 0.66 ms pass: 0.19 ms); the
 // conversion of a piece (about 10 us) is not worth a second buffer beside
 // its copy (1.2 ms at 64 MiB).
-constexpr size_t kRefStageBytes = (size_t)64 << 20, kRefStageMin = (size_t)1 << 20;
-
-void ref_stage_free(RefStage &st)
+cudaError_t ref_table_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
+                           Scratch &st, cudaStream_t s)
 {
-    cudaFree(st.p);
-    st = RefStage{};
-}
-
-cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
-                           RefStage &st, cudaStream_t s)
-{
+    constexpr size_t kLeast = (size_t)1 << 20;
     const size_t es = prec ? sizeof(double4) : sizeof(float4);
     const int planes = group == 3 ? 12 : 4;
-    const size_t plane_bytes = (size_t)rowsize * es, total = plane_bytes * planes;
-    const size_t want = total < kRefStageBytes ? total : kRefStageBytes;
-    if (st.bytes < want && !st.reduced) {
-        ref_stage_free(st);
-        size_t n = want;
-        // from the stream's pool: a first table costs no device-wide allocation
-        cudaError_t e = cudaMallocAsync(&st.p, n, s);
-        while (e == cudaErrorMemoryAllocation && n / 2 >= kRefStageMin) {
-            cudaGetLastError();                          // not left pending for the next launch check
-            n /= 2;
-            st.reduced = true;
-            e = cudaMallocAsync(&st.p, n, s);
-        }
-        if (e != cudaSuccess) {
-            st = RefStage{};
-            return e;
-        }
-        st.bytes = n;
-    }
-    const int step = (int)(st.bytes / plane_bytes);      // whole planes at a time; 0: pieces of one plane
-    const uint32_t piece = step ? rowsize : (uint32_t)(st.bytes / es);
+    const size_t total = (size_t)rowsize * es * planes, want = total < kScratchBytes ? total : kScratchBytes;
+    StreamMemory m{ s };
+    const cudaError_t e = scratch_reserve(m, st, want, want < kLeast ? want : kLeast);
+    if (e != cudaSuccess) return e;
     char *h = static_cast<char *>(host);
-    for (int p = 0; p < planes; p += step ? step : 1) {
-        const int np = step ? (planes - p < step ? planes - p : step) : 1;
-        for (uint32_t s0 = 0; s0 < rowsize;) {
-            const uint32_t s1 = rowsize - s0 > piece ? s0 + piece : rowsize;
-            const size_t bytes = (size_t)np * (s1 - s0) * es;
-            char *hp = h + (size_t)p * plane_bytes + (size_t)s0 * es;
-            cudaError_t e;
-            if (to_host) {
-                if ((e = launch_ref_piece<true>(G, links, st.p, prec, p, np, s0, s1, s)) != cudaSuccess) return e;
-                if ((e = cudaMemcpyAsync(hp, st.p, bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-            } else {
-                if ((e = cudaMemcpyAsync(st.p, hp, bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-                if ((e = launch_ref_piece<false>(G, links, st.p, prec, p, np, s0, s1, s)) != cudaSuccess) return e;
-            }
-            s0 = s1;
-        }
-    }
-    return cudaSuccess;
+    return table_pieces(
+        m, st.bytes, planes, rowsize, es, to_host,
+        [&](int p, int np, uint32_t s0, uint32_t s1) {
+            return to_host ? launch_ref_piece<true>(G, links, st.p, prec, p, np, s0, s1, s)
+                           : launch_ref_piece<false>(G, links, st.p, prec, p, np, s0, s1, s);
+        },
+        [&](size_t at, size_t n) {
+            return to_host ? cudaMemcpyAsync(h + at, st.p, n, cudaMemcpyDeviceToHost, s)
+                           : cudaMemcpyAsync(st.p, h + at, n, cudaMemcpyHostToDevice, s);
+        });
 }
 
 // final pass: one block sums the partials in a fixed order (deterministic)

@@ -9,6 +9,7 @@
 #include "../../include/qcdgpu_b200.h"
 #include <nvtx3/nvToolsExt.h>
 #include "qg_lattice.cuh"
+#include "qg_scratch.h"
 
 namespace qg {
 
@@ -39,18 +40,16 @@ enum InitKind { INIT_COLD = 0, INIT_GID = 1, INIT_HOT_REF = 2, INIT_HOT_PHILOX =
 cudaError_t launch_init(const Geom &G, void *links, int group, int prec, int kind, int dir,
                         const float4 *prns, uint32_t rowsize, uint2 key, cudaStream_t s);
 cudaError_t launch_gramschmidt(const Geom &G, void *links, int group, int prec, int fp64, cudaStream_t s);
-// the staging buffer of reference-layout table copies, kept by the owner of
-// the field (reduced: the wanted size was not free)
-struct RefStage {
-    void *p = nullptr;
-    size_t bytes = 0;
-    bool reduced = false;
-};
-void ref_stage_free(RefStage &st);
+// scratch kept by the owner of a field, for one call at a time: a link
+// table's pieces, the all-loops measurement.  scratch_free: nothing of it in
+// flight any more
+constexpr size_t kScratchBytes = (size_t)64 << 20;
+cudaError_t scratch_reserve(Scratch &st, size_t want, size_t least, cudaStream_t s);
+void scratch_free(Scratch &st);
 // the field as the reference-layout table in host memory (to_host), or that
-// table into the field; queued on s
-cudaError_t ref_stage_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
-                           RefStage &st, cudaStream_t s);
+// table into the field; queued on s (after an error nothing is in flight)
+cudaError_t ref_table_copy(const Geom &G, void *links, int group, int prec, uint32_t rowsize, void *host, bool to_host,
+                           Scratch &st, cudaStream_t s);
 
 // measurements: per-block partials into scratch, summed in a fixed order by
 // the last block into out (device or page-locked host memory); *ticket is a
@@ -91,14 +90,13 @@ cudaError_t launch_wilson_all(const Geom &G, const void *links, int group, int p
                               cudaStream_t s);
 // all loops in the time-line gauge (qg_wilson.cu): scratch of
 // wilson_lines_scratch bytes (0: a line does not fit, take
-// launch_wilson_all), slots of wilson_lines_slots doubles; out holds
+// launch_wilson_all; at most kScratchBytes); out holds
 // Rmax Tmax sums and then a flag, non-zero when a time line is too far from
 // unitary for its inverse to be taken (the sums are then not to be used)
-size_t wilson_lines_scratch(const Geom &G, int group, int Tmax);
-size_t wilson_lines_slots(int Rmax, int Tmax);
+size_t wilson_lines_scratch(const Geom &G, int group, int Rmax, int Tmax);
 cudaError_t launch_wilson_lines(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
-                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *slots,
-                                double *out, cudaStream_t s);
+                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *out,
+                                cudaStream_t s);
 cudaError_t launch_add_u64(uint64_t *p, uint64_t v, cudaStream_t s);
 // slab halo exchange: both sides of one (direction, parity) slice in one
 // launch; `unit` = 16-byte words per link-plane element, src / dst offsets

@@ -35,10 +35,11 @@
 
 namespace qg {
 
-constexpr int kSlots = 148 * 3;                         // blocks of k_loops: those resident at once
-size_t wilson_lines_slots(int Rmax, int Tmax) { return (size_t)kSlots * Rmax * Tmax; }
-
 namespace {
+
+constexpr int kSlots = 148 * 3;                         // blocks of k_loops: those resident at once
+// their sums, at the start of the scratch (256-byte multiples)
+size_t slots_doubles(int Rmax, int Tmax) { return ((size_t)kSlots * Rmax * Tmax + 31) / 32 * 32; }
 
 template <int NC> struct CM { CX<double> m[NC][NC]; };
 
@@ -558,8 +559,11 @@ cudaError_t loops(const Lines &L, double *slots, cudaStream_t s)
 
 template <int NC, typename Real>
 cudaError_t wilson_lines(const Field<Real> &U, const Geom &G, int Rmax, int Tmax, const double *params, int twist,
-                         double *scratch, size_t scratch_bytes, double *slots, double *out, cudaStream_t s)
+                         double *scratch, size_t scratch_bytes, double *out, cudaStream_t s)
 {
+    double *slots = scratch;
+    scratch += slots_doubles(Rmax, Tmax);
+    scratch_bytes -= slots_doubles(Rmax, Tmax) * sizeof(double);
     Lines L;
     L.G = G;
     L.Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
@@ -570,7 +574,7 @@ cudaError_t wilson_lines(const Field<Real> &U, const Geom &G, int Rmax, int Tmax
     double *flag = out + Rmax * Tmax;
     cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(double), s);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(slots, 0, wilson_lines_slots(Rmax, Tmax) * sizeof(double), s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(slots, 0, slots_doubles(Rmax, Tmax) * sizeof(double), s)) != cudaSuccess) return e;
     const uint32_t total = 3 * L.Vs;
     for (uint32_t g0 = 0; g0 < total;) {
         // whole lines, as many as the scratch holds (a chunk may run on from
@@ -607,29 +611,28 @@ cudaError_t wilson_lines(const Field<Real> &U, const Geom &G, int Rmax, int Tmax
 
 }  // namespace
 
-// the scratch of a chunk: at most kChunk bytes (the arrays are then read
-// from L2), no more than the lattice needs, 0 when one line does not fit
-size_t wilson_lines_scratch(const Geom &G, int group, int Tmax)
+// the sums of the blocks and the arrays of a chunk (read from L2 then): no
+// more than the lattice needs, 0 when one line does not fit
+size_t wilson_lines_scratch(const Geom &G, int group, int Rmax, int Tmax)
 {
-    constexpr size_t kChunk = (size_t)64 << 20;
-    const size_t col = column_bytes(G, group, Tmax);
+    const size_t col = column_bytes(G, group, Tmax), slots = slots_doubles(Rmax, Tmax) * sizeof(double);
     const size_t line = col * std::max(G.n[0], std::max(G.n[1], G.n[2]));
     const size_t all = col * 3 * ((size_t)G.n[0] * G.n[1] * G.n[2]);
-    return line > kChunk ? 0 : std::min(kChunk, all);
+    return slots + line > kScratchBytes ? 0 : std::min(kScratchBytes, slots + all);
 }
 
 cudaError_t launch_wilson_lines(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
-                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *slots,
-                                double *out, cudaStream_t s)
+                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *out,
+                                cudaStream_t s)
 {
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        return group == 3 ? wilson_lines<3, double>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, slots, out, s)
-                          : wilson_lines<2, double>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, slots, out, s);
+        return group == 3 ? wilson_lines<3, double>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s)
+                          : wilson_lines<2, double>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s);
     }
     Field<float> U{ (float4 *)links, G.pstride };
-    return group == 3 ? wilson_lines<3, float>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, slots, out, s)
-                      : wilson_lines<2, float>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, slots, out, s);
+    return group == 3 ? wilson_lines<3, float>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s)
+                      : wilson_lines<2, float>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s);
 }
 
 }  // namespace qg
