@@ -660,8 +660,13 @@ cudaError_t launch_after(void (*kern)(Field<Real>, Geom, PhaseArgs), unsigned nb
 // the first slots come free: SU(3) FP32 12^3 x 8 overrelaxation 3.2 us
 // without, 4.2 with it, 4^4 2.65 / 2.31).
 template <int NC, typename Real, int PM, bool OR, int MU, int SP>
-bool try_split(const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStream_t s, cudaError_t &e)
+unsigned split_limit(unsigned nb)
 {
+    constexpr bool kF32 = sizeof(Real) == 4;
+    if constexpr (NC == 2 && OR) return kF32 ? 128 : 512;
+    // more than 64 warps per SM would hold: the driver is not asked (it would
+    // load a kernel that a large lattice never launches, 0.1 ms each)
+    if (nb > 148u * (64 / SP) * 3 / 4) return 0;
     static const int per_sm = [] {
         int n = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_phase_split<NC, Real, PM, OR, MU, SP>, 32 * SP, 0) !=
@@ -671,17 +676,23 @@ bool try_split(const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStre
         }
         return n;
     }();
-    const unsigned nb = (a.t_end - a.t_begin + 31) / 32, resident = 148u * per_sm;
-    constexpr bool kF32 = sizeof(Real) == 4;
-    unsigned limit;
-    if (NC == 2 && OR) limit = SP == 6 ? (kF32 ? 128 : 512) : 0;
-    else if (SP == 6) limit = NC == 3 ? resident * 3 / 4 : resident * 3 / 5;
-    else if (NC == 2 && !kF32) limit = 0;
-    else limit = (OR && kF32) || (!OR && PM == 0) ? resident / 2 : resident * 3 / 4;
-    if (nb > limit) return false;
-    const bool early = a.after_phase && ((!OR && PM == 1) || nb <= 74);
-    e = launch_after(k_phase_split<NC, Real, PM, OR, MU, SP>, nb, 32 * SP, early, U, G, a, s);
-    return true;
+    const unsigned resident = 148u * per_sm;
+    if (SP == 6) return NC == 3 ? resident * 3 / 4 : resident * 3 / 5;
+    return (OR && kF32) || (!OR && PM == 0) ? resident / 2 : resident * 3 / 4;
+}
+
+template <int NC, typename Real, int PM, bool OR, int MU, int SP>
+bool try_split(const Field<Real> &U, const Geom &G, const PhaseArgs &a, cudaStream_t s, cudaError_t &e)
+{
+    if constexpr (SP == 3 && NC == 2 && (OR || sizeof(Real) == 8)) {
+        return false;
+    } else {
+        const unsigned nb = (a.t_end - a.t_begin + 31) / 32;
+        if (nb > split_limit<NC, Real, PM, OR, MU, SP>(nb)) return false;
+        const bool early = a.after_phase && ((!OR && PM == 1) || nb <= 74);
+        e = launch_after(k_phase_split<NC, Real, PM, OR, MU, SP>, nb, 32 * SP, early, U, G, a, s);
+        return true;
+    }
 }
 
 template <typename Real>
