@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # -fmad=false: every fused multiply-add in the kernels is an explicit fma()
 # in a fixed order, so results do not depend on the compiler's contraction
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC", "-I" + INCLUDE]
-CUDA_SOURCES = ["qg_update_f32.cu", "qg_update_f64.cu", "qg_fields.cu", "qg_wilson.cu", "qg_ranlux.cu", "qg_capi.cu",
+CUDA_SOURCES = ["qg_update_f32.cu", "qg_update_f64.cu", "qg_fields.cu", "qg_ranlux.cu", "qg_capi.cu",
                 "qg_noalloc.cu", "qg_batch.cu",
                 "qg_learned.cu"]
 LIB_HOST_SOURCES = ["qg_host.cpp", "qg_state.cpp", "qg_results.cpp"]          # C++ host code linked into the library

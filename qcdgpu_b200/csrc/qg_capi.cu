@@ -1391,7 +1391,7 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
     const qg_config &f = c->cfg;
     int tw = !(f.phi == 0.0 && f.omega == 0.0);
     const int nl = Rmax * Tmax;
-    // The time-line gauge (qg_wilson.cu; FP64 products whatever fp64_products
+    // The time-line gauge (qg_wilson.cuh; FP64 products whatever fp64_products
     // says) costs a preparation and little per loop, the column kernel two
     // products per loop and R (R - 1) / 2 for the lines.  At SU(3) 32^4 FP32
     // the gauge takes 1.27 ms + 0.19 ms per R, the column kernel 0.24 / 0.18

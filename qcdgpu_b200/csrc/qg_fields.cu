@@ -4,6 +4,7 @@
 // deterministic two-pass FP64 reductions.
 #include "qg_internal.h"
 #include "qg_observe.cuh"
+#include "qg_wilson.cuh"
 
 namespace qg {
 

@@ -88,7 +88,7 @@ size_t wilson_all_partials(int nbx, int Rmax);
 cudaError_t launch_wilson_all(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
                               int fp64_products, const double *params, int twist, double *partials, double *out,
                               cudaStream_t s);
-// all loops in the time-line gauge (qg_wilson.cu): scratch of
+// all loops in the time-line gauge (qg_wilson.cuh): scratch of
 // wilson_lines_scratch bytes (0: a line does not fit, take
 // launch_wilson_all; at most kScratchBytes); out holds
 // Rmax Tmax sums and then a flag, non-zero when a time line is too far from
