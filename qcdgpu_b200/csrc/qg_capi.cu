@@ -72,7 +72,10 @@ struct qg_ctx {
     bool slab = false;
     int slab_x0 = 0, slab_n1 = 0;
     unsigned long long *d_bad = nullptr;   // qg_field_check counter
-    Scratch scratch;                // link table copies and the all-loops measurement (lazy)
+    Scratch scratch;                // link table copies (lazy)
+    Scratch loops;                  // the all-loops measurement's second part, where `scratch` has no room (lazy)
+    double *d_wpart = nullptr;      // the same, column kernel (lazy)
+    int wpart_rmax = 0;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_phase[8] = {};
     // learned-proposal Metropolis (qg_net_*, qg_mh_*)
@@ -241,6 +244,8 @@ extern "C" int qg_destroy(qg_ctx *c)
     cudaFree(c->d_fpart); cudaFree(c->d_ppart); cudaFree(c->d_pout); cudaFree(c->d_sites);
     cudaFree(c->d_bad);
     scratch_free(c->scratch);
+    scratch_free(c->loops);
+    cudaFree(c->d_wpart);
     if (c->h_results) cudaFreeHost(c->h_results);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_ring) cudaFreeHost(c->h_ring);
@@ -1404,13 +1409,25 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
     // where a line is larger than the scratch, the scratch is not free, or a
     // time line is too far from unitary to be inverted.
     const bool gauge = nl >= (c->G.V <= 4096 ? 25 : (f.precision || fp64_products) ? 16 : 32);
-    const size_t lines = gauge ? wilson_lines_scratch(c->G, f.group, Rmax, Tmax) : 0;
+    int nparts = 0;
+    const size_t part = gauge ? wilson_lines_scratch(c->G, f.group, Rmax, Tmax, nparts) : 0;
     double *d_wout = c->d_results + 64;
-    cudaError_t e = lines ? scratch_reserve(c->scratch, lines, lines, c->stream) : cudaErrorMemoryAllocation;
+    // the parts: both in the table scratch where it has room for them (a table
+    // of 64 MiB has moved), else the first there and the second of its own:
+    // one mapping of the pool each, and none is given back (a buffer of 64 MiB
+    // is two mappings, and growing the scratch to it unmaps one)
+    cudaError_t e = part ? cudaSuccess : cudaErrorMemoryAllocation;
+    const bool both = nparts == 2 && c->scratch.bytes >= 2 * part;
+    if (e == cudaSuccess && !both) e = scratch_reserve(c->scratch, part, c->stream);
+    if (e == cudaSuccess && !both && nparts == 2) e = scratch_reserve(c->loops, part, c->stream);
     if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "wilson scratch");
     if (e == cudaSuccess) {
-        QG_CK(launch_wilson_lines(c->G, c->links, f.group, f.precision, Rmax, Tmax, c->d_params, tw,
-                                  (double *)c->scratch.p, lines, d_wout, c->stream), "wilson all");
+        double *const first = static_cast<double *>(c->scratch.p);
+        double *const parts[2] = { first, nparts == 1 ? nullptr
+                                          : both      ? first + part / sizeof(double)
+                                                      : static_cast<double *>(c->loops.p) };
+        QG_CK(launch_wilson_lines(c->G, c->links, f.group, f.precision, Rmax, Tmax, c->d_params, tw, parts, part, d_wout,
+                                  c->stream), "wilson all");
         double h[kLoopResults];
         QG_CK(cudaMemcpyAsync(h, d_wout, (size_t)(nl + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
               "wilson copy");
@@ -1420,10 +1437,16 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
             return QG_OK;
         }
     }
-    const size_t cols = wilson_all_partials(wilson_all_blocks(c->G), Rmax) * sizeof(double);
-    QG_CK(scratch_reserve(c->scratch, cols, cols, c->stream), "wilson scratch");
+    if (c->wpart_rmax < Rmax) {
+        cudaFree(c->d_wpart);
+        c->d_wpart = nullptr;
+        c->wpart_rmax = 0;
+        QG_CK(cudaMalloc(&c->d_wpart, wilson_all_partials(wilson_all_blocks(c->G), Rmax) * sizeof(double)),
+              "wilson scratch");
+        c->wpart_rmax = Rmax;
+    }
     QG_CK(launch_wilson_all(c->G, c->links, f.group, f.precision, Rmax, Tmax, fp64_products, c->d_params, tw,
-                            (double *)c->scratch.p, d_wout, c->stream), "wilson all");
+                            c->d_wpart, d_wout, c->stream), "wilson all");
     QG_CK(cudaMemcpyAsync(out, d_wout, (size_t)nl * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
           "wilson copy");
     QG_CK(cudaStreamSynchronize(c->stream), "wilson sync");

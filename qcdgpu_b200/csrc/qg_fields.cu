@@ -364,10 +364,10 @@ struct StreamMemory {
 };
 }  // namespace
 
-cudaError_t scratch_reserve(Scratch &st, size_t want, size_t least, cudaStream_t s)
+cudaError_t scratch_reserve(Scratch &st, size_t want, cudaStream_t s)
 {
     StreamMemory m{ s };
-    return scratch_reserve(m, st, want, least);
+    return scratch_reserve(m, st, want, want);
 }
 
 void scratch_free(Scratch &st)

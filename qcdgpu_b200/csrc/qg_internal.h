@@ -40,11 +40,11 @@ enum InitKind { INIT_COLD = 0, INIT_GID = 1, INIT_HOT_REF = 2, INIT_HOT_PHILOX =
 cudaError_t launch_init(const Geom &G, void *links, int group, int prec, int kind, int dir,
                         const float4 *prns, uint32_t rowsize, uint2 key, cudaStream_t s);
 cudaError_t launch_gramschmidt(const Geom &G, void *links, int group, int prec, int fp64, cudaStream_t s);
-// scratch kept by the owner of a field, for one call at a time: a link
-// table's pieces, the all-loops measurement.  scratch_free: nothing of it in
-// flight any more
-constexpr size_t kScratchBytes = (size_t)64 << 20;
-cudaError_t scratch_reserve(Scratch &st, size_t want, size_t least, cudaStream_t s);
+// scratch kept by the owner of a field, for one call at a time.
+// scratch_reserve: all of `want`, from the pool of stream s (which maps 32 MiB
+// at a time); scratch_free: nothing of it in flight any more
+constexpr size_t kScratchPart = (size_t)32 << 20, kScratchBytes = 2 * kScratchPart;
+cudaError_t scratch_reserve(Scratch &st, size_t want, cudaStream_t s);
 void scratch_free(Scratch &st);
 // the field as the reference-layout table in host memory (to_host), or that
 // table into the field; queued on s (after an error nothing is in flight)
@@ -88,15 +88,15 @@ size_t wilson_all_partials(int nbx, int Rmax);
 cudaError_t launch_wilson_all(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
                               int fp64_products, const double *params, int twist, double *partials, double *out,
                               cudaStream_t s);
-// all loops in the time-line gauge (qg_wilson.cuh): scratch of
-// wilson_lines_scratch bytes (0: a line does not fit, take
-// launch_wilson_all; at most kScratchBytes); out holds
+// all loops in the time-line gauge (qg_wilson.cuh): scratch of 1 or 2 parts
+// (parts[1] null: 1) of wilson_lines_scratch bytes each (0: a line does not
+// fit, take launch_wilson_all; at most kScratchPart); out holds
 // Rmax Tmax sums and then a flag, non-zero when a time line is too far from
 // unitary for its inverse to be taken (the sums are then not to be used)
-size_t wilson_lines_scratch(const Geom &G, int group, int Rmax, int Tmax);
+size_t wilson_lines_scratch(const Geom &G, int group, int Rmax, int Tmax, int &parts);
 cudaError_t launch_wilson_lines(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
-                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *out,
-                                cudaStream_t s);
+                                const double *params, int twist, double *const parts[2], size_t part_bytes,
+                                double *out, cudaStream_t s);
 cudaError_t launch_add_u64(uint64_t *p, uint64_t v, cudaStream_t s);
 // slab halo exchange: both sides of one (direction, parity) slice in one
 // launch; `unit` = 16-byte words per link-plane element, src / dst offsets

@@ -116,17 +116,19 @@ __device__ __forceinline__ CM<NC> cinv(const CM<NC> &a, double &det2)
 // line along i), columns [g0, g0 + ncol) in the scratch arrays
 // [column][t / 8][component][t % 8]: a component is a fixed distance from
 // the first (no address arithmetic per component) and eight lanes share two
-// sectors.  NT1 >= N4 + Tmax, a multiple of 8.
+// sectors.  NT1 >= N4 + Tmax, a multiple of 8.  Columns from `cut` on lie in
+// the second part of the scratch (`jump` further); a line lies in one part.
 struct Lines {
     Geom G;
-    uint32_t Vs, g0, ncol;
+    uint32_t Vs, g0, ncol, cut;
     int NT1, Rmax, Tmax;
+    ptrdiff_t jump;
     double *V, *K, *F;
 };
 template <int NC>
-__device__ __forceinline__ size_t at_index(const Lines &L, uint32_t col, int t)
+__device__ __forceinline__ ptrdiff_t at_index(const Lines &L, uint32_t col, int t)
 {
-    return ((size_t)col * (L.NT1 / 8) + t / 8) * (2 * NC * NC * 8) + t % 8;
+    return ((ptrdiff_t)col * (L.NT1 / 8) + t / 8) * (2 * NC * NC * 8) + t % 8 + (col < L.cut ? 0 : L.jump);
 }
 
 __device__ __forceinline__ Crd column(const Lines &L, uint32_t g, int &i, int &x)
@@ -347,8 +349,8 @@ __global__ void __launch_bounds__(128) k_line_links(Field<Real> U, Lines L, cons
     int i, x;
     Crd c = column(L, L.g0 + col, i, x);
     const int ni = i == 0 ? L.G.n[0] : i == 1 ? L.G.n[1] : L.G.n[2];
-    const size_t at = at_index<NC>(L, col, t);
-    const size_t nx = at_index<NC>(L, x + 1 == ni ? col - (uint32_t)x : col + 1, t);     // column x + i of the line
+    const ptrdiff_t at = at_index<NC>(L, col, t);
+    const ptrdiff_t nx = at_index<NC>(L, x + 1 == ni ? col - (uint32_t)x : col + 1, t);     // column x + i of the line
     c.t = t % nt;
     const CM<NC> u = link_cm<NC, Real>(U, L.G, c, i, params, TW ? twist : 0);
     const CM<NC> v = load_soa<NC>(L.V + at), w = load_soa<NC>(L.V + nx);
@@ -431,7 +433,7 @@ __global__ void __launch_bounds__(kLoopThreads, 3) k_loops(Lines L, int cols, in
             int i;
             column(L, L.g0 + col, i, x);
             ni = i == 0 ? L.G.n[0] : i == 1 ? L.G.n[1] : L.G.n[2];
-            const size_t o = at_index<NC>(L, col, t);
+            const ptrdiff_t o = at_index<NC>(L, col, t);
             at = link + o;
             CM<NC> v = load_soa<NC>(L.V + o);
             k = load_soa<NC>(at);
@@ -562,40 +564,45 @@ cudaError_t loops(const Lines &L, double *slots, cudaStream_t s)
 
 template <int NC, typename Real>
 cudaError_t wilson_lines(const Field<Real> &U, const Geom &G, int Rmax, int Tmax, const double *params, int twist,
-                         double *scratch, size_t scratch_bytes, double *out, cudaStream_t s)
+                         double *const parts[2], size_t part_bytes, double *out, cudaStream_t s)
 {
-    double *slots = scratch;
-    scratch += slots_doubles(Rmax, Tmax);
-    scratch_bytes -= slots_doubles(Rmax, Tmax) * sizeof(double);
+    const size_t head = slots_doubles(Rmax, Tmax);      // left free in the second part
+    double *slots = parts[0];
     Lines L;
     L.G = G;
     L.Vs = (uint32_t)G.n[0] * G.n[1] * G.n[2];
     L.Rmax = Rmax;
     L.Tmax = Tmax;
     L.NT1 = padded_nt(G, Tmax);
-    const uint32_t maxcol = (uint32_t)std::min<size_t>(scratch_bytes / column_bytes(G, NC, Tmax), (size_t)3 * L.Vs);
+    const uint32_t total = 3 * L.Vs;
+    const size_t column = (size_t)2 * NC * NC * L.NT1;
+    const uint32_t maxcol = (uint32_t)std::min<size_t>((part_bytes / sizeof(double) - head) / (3 * column), total);
+    L.V = parts[0] + head;
+    L.K = L.V + maxcol * column;
+    L.F = L.K + maxcol * column;
     double *flag = out + Rmax * Tmax;
     cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(double), s);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(slots, 0, slots_doubles(Rmax, Tmax) * sizeof(double), s)) != cudaSuccess) return e;
-    const uint32_t total = 3 * L.Vs;
-    for (uint32_t g0 = 0; g0 < total;) {
-        // whole lines, as many as the scratch holds (a chunk may run on from
-        // one direction's lines to the next one's)
-        uint32_t g1 = g0;
-        while (g1 < total) {
-            const int i = (int)(g1 / L.Vs);
-            const uint32_t ni = (uint32_t)G.n[i], room = maxcol - (g1 - g0), left = (uint32_t)(i + 1) * L.Vs - g1;
+    // whole lines from column g on, as many as a part holds (they may run on
+    // from one direction's lines to the next one's)
+    auto part_end = [&](uint32_t g) {
+        const uint32_t g0 = g;
+        while (g < total) {
+            const int i = (int)(g / L.Vs);
+            const uint32_t ni = (uint32_t)G.n[i], room = maxcol - (g - g0), left = (uint32_t)(i + 1) * L.Vs - g;
             const uint32_t take = std::min(room / ni * ni, left);
-            g1 += take;
+            g += take;
             if (take < left) break;
         }
+        return g;
+    };
+    for (uint32_t g0 = 0; g0 < total;) {
+        const uint32_t gc = part_end(g0), g1 = parts[1] ? part_end(gc) : gc;
         L.g0 = g0;
         L.ncol = g1 - g0;
-        const size_t n = (size_t)2 * NC * NC * L.ncol * L.NT1;
-        L.V = scratch;
-        L.K = L.V + n;
-        L.F = L.K + n;
+        L.cut = gc - g0;
+        L.jump = parts[1] ? parts[1] - parts[0] - (ptrdiff_t)(L.cut * column) : 0;
         const int nwork = std::min(L.NT1 / kSeg, kTLSegs<NC, Real>);
         k_time_lines<NC, Real><<<(L.ncol + kTLCols - 1) / kTLCols, kTLCols * NC * nwork, 0, s>>>(U, L);
         const unsigned nb = (unsigned)(((size_t)L.ncol * L.NT1 + 127) / 128);
@@ -614,28 +621,30 @@ cudaError_t wilson_lines(const Field<Real> &U, const Geom &G, int Rmax, int Tmax
 
 }  // namespace
 
-// the sums of the blocks and the arrays of a chunk (read from L2 then): no
-// more than the lattice needs, 0 when one line does not fit
-size_t wilson_lines_scratch(const Geom &G, int group, int Rmax, int Tmax)
+// the sums of the blocks and the arrays of a chunk (read from L2 then), in one
+// part where the lattice needs no more, else in two: 0 when one line does
+// not fit a part
+size_t wilson_lines_scratch(const Geom &G, int group, int Rmax, int Tmax, int &parts)
 {
     const size_t col = column_bytes(G, group, Tmax), slots = slots_doubles(Rmax, Tmax) * sizeof(double);
     const size_t line = col * std::max(G.n[0], std::max(G.n[1], G.n[2]));
-    const size_t all = col * 3 * ((size_t)G.n[0] * G.n[1] * G.n[2]);
-    return slots + line > kScratchBytes ? 0 : std::min(kScratchBytes, slots + all);
+    const size_t all = slots + col * 3 * ((size_t)G.n[0] * G.n[1] * G.n[2]);
+    parts = all > kScratchPart ? 2 : 1;
+    return slots + line > kScratchPart ? 0 : std::min(kScratchPart, all);
 }
 
 cudaError_t launch_wilson_lines(const Geom &G, const void *links, int group, int prec, int Rmax, int Tmax,
-                                const double *params, int twist, double *scratch, size_t scratch_bytes, double *out,
-                                cudaStream_t s)
+                                const double *params, int twist, double *const parts[2], size_t part_bytes,
+                                double *out, cudaStream_t s)
 {
     if (prec) {
         Field<double> U{ (double4 *)links, G.pstride };
-        return group == 3 ? wilson_lines<3, double>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s)
-                          : wilson_lines<2, double>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s);
+        return group == 3 ? wilson_lines<3, double>(U, G, Rmax, Tmax, params, twist, parts, part_bytes, out, s)
+                          : wilson_lines<2, double>(U, G, Rmax, Tmax, params, twist, parts, part_bytes, out, s);
     }
     Field<float> U{ (float4 *)links, G.pstride };
-    return group == 3 ? wilson_lines<3, float>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s)
-                      : wilson_lines<2, float>(U, G, Rmax, Tmax, params, twist, scratch, scratch_bytes, out, s);
+    return group == 3 ? wilson_lines<3, float>(U, G, Rmax, Tmax, params, twist, parts, part_bytes, out, s)
+                      : wilson_lines<2, float>(U, G, Rmax, Tmax, params, twist, parts, part_bytes, out, s);
 }
 
 }  // namespace qg

@@ -61,6 +61,19 @@ def test_repeated_calls_of_other_extents_share_the_scratch():
     L.close()
 
 
+@pytest.mark.parametrize("group,size,precision", [(3, (24, 24, 24, 22), 1), (3, (20, 18, 22, 14), 0), (2, (6, 10, 8, 12), 1)])
+def test_loops_do_not_depend_on_where_the_scratch_lies(group, size, precision):
+    """the same bits in a context that has moved no table, and in one that has (the scratch then holds both parts,
+    the first one, or all there is)"""
+    A, B = lattice(group, size, precision, sweeps=1), lattice(group, size, precision, sweeps=1)
+    t = B.download()
+    a, b = A.wilson_all(5, 6), B.wilson_all(5, 6)
+    assert np.array_equal(a, b) and np.array_equal(B.wilson_all(5, 6), a)
+    assert np.array_equal(A.download(), t) and np.array_equal(A.wilson_all(5, 6), a)
+    A.close()
+    B.close()
+
+
 @pytest.mark.parametrize("twist", [(0.0, 0.0), (0.4, 0.9)])
 def test_links_off_su3(twist):
     """rows scaled by up to 3 %: the loops are products of the stored links,
