@@ -1397,18 +1397,27 @@ extern "C" int qg_measure_wilson_all(qg_ctx *c, int Rmax, int Tmax, int fp64_pro
     int tw = !(f.phi == 0.0 && f.omega == 0.0);
     const int nl = Rmax * Tmax;
     // The time-line gauge (qg_wilson.cuh; FP64 products whatever fp64_products
-    // says) costs a preparation and little per loop, the column kernel two
-    // products per loop and R (R - 1) / 2 for the lines.  At SU(3) 32^4 FP32
-    // the gauge takes 1.27 ms + 0.19 ms per R, the column kernel 0.24 / 0.18
-    // ms (FP64 / FP32 products) for 1 x 1, 1.50 / 0.80 for 1 x 8, 2.11 / 1.27
-    // for 8 x 1 and 12.8 / 5.6 for 8 x 8: they cross near R T = 16 with FP64
-    // products (4 x 4: 1.99 against 2.46 ms) and 32 with FP32 ones (5 x 5:
-    // 2.34 against 2.07, 4 x 7: 2.11 against 2.37).  On up to 8^4 sites both
-    // are latency (4^4, 4 x 4: 53 us either way; 8^4, 5 x 5: 65 against 89 us
-    // whatever the products).  The column kernel also
-    // where a line is larger than the scratch, the scratch is not free, or a
-    // time line is too far from unitary to be inverted.
-    const bool gauge = nl >= (c->G.V <= 4096 ? 25 : (f.precision || fp64_products) ? 16 : 32);
+    // says) costs a preparation and so much per R, both for the padded time
+    // extents of its arrays; the column kernel costs two products per loop.  At
+    // SU(3) 32^4 FP32 the gauge takes 1.27 ms + 0.19 ms per R, the column
+    // kernel 0.24 / 0.18 ms (FP64 / FP32 products) for 1 x 1, 1.50 / 0.80 for
+    // 1 x 8, 2.11 / 1.27 for 8 x 1 and 12.8 / 5.6 for 8 x 8.  The factors are
+    // the least with which no shape of 1600 measured (N4 = 4 .. 96, up to 32^4;
+    // R T <= 144) is more than 5 % slower than in the column kernel: a short N4
+    // pads most (32^3 x 6, FP32 products, 6 x 6: 891 against 671 us, 4 x 4 with
+    // FP64 ones 27 %, both in the column kernel by this rule).  SU(2) in the
+    // gauge from R T = 16 (FP64 products) and 32 on is slower at none of 700
+    // (32^4 FP32 4 x 4: 0.82 against 1.12 ms; 24^3 x 6 8 x 4, FP32 products: 0.18
+    // against 0.23).  On up to 8^4 sites both are latency (8^4, 5 x 5: 65 against
+    // 89 us whatever the products).  The column kernel also where a line is
+    // larger than the scratch, the scratch is not free, or a time line is too far
+    // from unitary to be inverted.
+    const int wide = f.precision || fp64_products, n4 = c->G.n[3];
+    const int padded = (n4 + Tmax + 7) / 8 * 8 + (n4 + 7) / 8 * 8;          // of D and E
+    const bool gauge = c->G.V <= 4096 ? nl >= 25
+                       : f.group == 2 ? nl >= (wide ? 16 : 32)
+                       : wide         ? 4 * n4 * nl >= padded * (Rmax + 20)
+                                      : 10 * n4 * nl >= 8 * padded * (Rmax + 10);
     int nparts = 0;
     const size_t part = gauge ? wilson_lines_scratch(c->G, f.group, Rmax, Tmax, nparts) : 0;
     double *d_wout = c->d_results + 64;

@@ -43,6 +43,8 @@ def check(L, Rmax, Tmax, loops, fp64=True):
     (2, (10, 10, 10, 66), 1, (10, 3)),       # time extents split into windows, the last one ragged
     (3, (2, 2, 2, 150), 0, (2, 16)),
     (3, (24, 24, 24, 22), 0, (6, 3)),        # several chunks of lines, breaking inside a direction
+    (3, (10, 10, 10, 6), 1, (6, 4)),         # short time extents: the column kernel, then the gauge
+    (3, (10, 10, 10, 6), 1, (6, 6)),
 ])
 def test_loops_equal_the_single_loops(group, size, precision, rt):
     L = lattice(group, size, precision)
