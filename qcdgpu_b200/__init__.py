@@ -592,7 +592,7 @@ class Lattice:
     def sweep_phase_times(self, n=20):
         """qg_sweep_phase_times: n sweeps of the qg_sweep chain, returning the
         mean (heatbath phase, overrelaxation phase, whole sweep) durations
-        in ms inside the sweep graph"""
+        in ms, in a sweep graph whose phases run one after another"""
         hb, orx, sw = ctypes.c_double(), ctypes.c_double(), ctypes.c_double()
         self._ck(self.lib.qg_sweep_phase_times(self.ctx, n, ctypes.byref(hb), ctypes.byref(orx), ctypes.byref(sw)),
                  "qg_sweep_phase_times")

@@ -716,6 +716,56 @@ extern "C" int qg_profile_kernels(qg_ctx *c, int reps, double *mean_ms, double *
     return QG_OK;
 }
 
+// ms of one phase of a.variant, launched as the sweep graph launches it: up to
+// 2^16 links in a graph of its own (a phase may be launched early there, and
+// takes less than a launch by the host: SU(2) FP64 8^4, 2.7 and 4.9 us in shapes
+// 0 and 1, both 6.9 us one launch after another), else in the stream
+static cudaError_t time_shape(qg_ctx *c, PhaseArgs a, int kind, int reps, cudaEvent_t e0, cudaEvent_t e1, float *ms)
+{
+    cudaError_t e = cudaSuccess;
+    if (a.t_end - a.t_begin > 65536) {
+        // one untimed launch, then reps timed ones over the 8 phase classes
+        for (int r = -1; r < reps && e == cudaSuccess; r++) {
+            if (r == 0) cudaEventRecord(e0, c->stream);
+            a.parity = (r + 1) & 1;
+            a.dir = ((r + 1) >> 1) & 3;
+            e = launch_phase(c, a);
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
+        *ms /= (float)reps;
+        return e;
+    }
+    const int n = reps < 64 ? (reps + 7) / 8 * 8 : 64, timed = std::max(3, reps / n);
+    const bool batches = kind == QG_UPDATE_HEATBATH && a.prn_mode == QG_PRNG_RANLUX && !c->rl_look_enabled;
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t gx = nullptr;
+    if ((e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
+    for (int k = 0; k < n && e == cudaSuccess; k++) {
+        a.parity = 1 - ((k >> 2) & 1);
+        a.dir = k & 3;
+        a.after_phase = k > 0 && !batches;
+        e = launch_phase(c, a);
+    }
+    const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&gx, g, 0);
+    *ms = 1e30f;
+    for (int r = -1; r < timed && e == cudaSuccess; r++) {       // one untimed launch first
+        float t = 0;
+        if ((e = cudaEventRecord(e0, c->stream)) != cudaSuccess) break;
+        if ((e = cudaGraphLaunch(gx, c->stream)) != cudaSuccess) break;
+        if ((e = cudaEventRecord(e1, c->stream)) != cudaSuccess) break;
+        if ((e = cudaEventSynchronize(e1)) != cudaSuccess) break;
+        if ((e = cudaEventElapsedTime(&t, e0, e1)) != cudaSuccess) break;
+        if (r >= 0 && t / n < *ms) *ms = t / n;
+    }
+    if (gx) cudaGraphExecDestroy(gx);
+    if (g) cudaGraphDestroy(g);
+    return e;
+}
+
 // times each launch shape of the heatbath and overrelaxation phase kernels
 // on the live field (restored afterwards, PRN counters untouched) and keeps
 // the fastest per kind
@@ -738,18 +788,9 @@ extern "C" int qg_tune(qg_ctx *c, int reps, float *times_ms)
         for (int kind = 0; kind < 2 && e == cudaSuccess; kind++) {
             PhaseArgs a = phase_args(c, 0, 0, kind, 0);
             a.variant = v;
-            // one untimed launch, then reps timed ones over the 8 phase classes
-            for (int r = -1; r < reps && e == cudaSuccess; r++) {
-                if (r == 0) cudaEventRecord(e0, c->stream);
-                a.parity = (r + 1) & 1;
-                a.dir = ((r + 1) >> 1) & 3;
-                e = launch_phase(c, a);
-            }
-            cudaEventRecord(e1, c->stream);
-            cudaEventSynchronize(e1);
             float ms = 0;
-            cudaEventElapsedTime(&ms, e0, e1);
-            ms /= reps;
+            e = time_shape(c, a, kind, reps, e0, e1, &ms);
+            if (e != cudaSuccess) break;
             if (times_ms) times_ms[2 * v + kind] = ms;
             if (ms < best[kind]) { best[kind] = ms; arg[kind] = v; }
         }
@@ -1062,11 +1103,11 @@ extern "C" int qg_sweep(qg_ctx *c, int nsweeps)
     return QG_OK;
 }
 
-// nsweeps sweeps of the qg_sweep chain (Philox stream, same launches and
+// nsweeps sweeps of the qg_sweep chain (Philox stream, same kernels and
 // reunitarisation cadence) captured as one graph with an event node before
 // and after every phase launch and around the whole: the mean duration of a
-// heatbath and of an overrelaxation phase as they run inside the sweep
-// graph, and of a whole sweep in that graph
+// heatbath and of an overrelaxation phase each by itself (no early launches:
+// the events keep them apart), and of a whole sweep in that graph
 extern "C" int qg_sweep_phase_times(qg_ctx *c, int nsweeps, double *ms_heatbath, double *ms_overrelax,
                                     double *ms_sweep)
 {
