@@ -773,7 +773,8 @@ __global__ void __launch_bounds__(128) k_wilson(Field<Real> U, Geom G, int R, in
 // the loop is Re Tr((L_t S(t+T)) (S(t) L_t')^+) with the time lines L_t =
 // L_t^T(x), L_t' = L_t^T(x+R i): (R-1) + 2 (T-1) + 2 products per (x, i, t)
 // against 2 (R-1) + (T-1) + 3 and (T-1)/3 of k_wilson, and half the link
-// loads and row-3 rebuilds.  Bound by the FP64 pipe.
+// loads and row-3 rebuilds.  Bound by the L1 data path (74 % busy at 32^4 with
+// FP64 links, the FP64 pipe 42 %).
 template <int NC, typename Real, bool TW>
 __global__ void __launch_bounds__(128) k_wilson_line(Field<Real> U, Geom G, int R, int T, int cols,
                                                       const double *params, int twist, double *partials,

@@ -647,11 +647,11 @@ cudaError_t launch_after(void (*kern)(Field<Real>, Geom, PhaseArgs), unsigned nb
 // RANLUX batches, whose generator wants the SMs too: 1/2; not the SU(2) FP64
 // heatbath); the SU(2) overrelaxation, little more than its loads, up to 128
 // blocks (FP64: 512).  Measured in the sweep graph, us a phase, heatbath /
-// overrelaxation, one thread per link -> split:
-//   SU(3) FP32  8^4   9.4 / 4.8 -> 6.6 / 2.7    16^3 x 8   9.7 / 4.9 -> 8.4 / 4.4
-//   SU(3) FP64  8^4  11.5 / 6.2 -> 7.0 / 3.6    16^3 x 8  11.9 / 6.4 -> 9.8 / 6.6
-//   SU(2) FP32  8^4   4.9 / 2.4 -> 2.6 / 1.5    16^4       5.1       -> 4.5
-//   SU(2) FP64  8^4   4.9 / 2.7 -> 2.7 / 1.7    16^3 x 8   5.2 / 2.9 -> 4.1 / 2.8
+// overrelaxation, one thread per link (the faster of its forms) -> split:
+//   SU(3) FP32  8^4   8.9 / 4.4 -> 6.8 / 2.8    16^3 x 8   9.8 / 5.1 -> 8.5 / 4.2
+//   SU(3) FP64  8^4  11.1 / 5.8 -> 6.9 / 3.9    12^3 x 8  11.8 / 6.4 -> 7.9 / 4.8
+//   SU(2) FP32  8^4   4.1 / 2.0 -> 2.6 / 1.5    16^4       4.9       -> 4.4
+//   SU(2) FP64  8^4   4.7 / 2.7 -> 2.7 / 1.7    16^3 x 8   5.1 / 2.8 -> 4.1 / 2.9
 // and beyond the limits: SU(3) FP32 16^4 10.9 / 5.3 against 13.1 / 6.2 with
 // SP = 3, FP64 14.3 / 8.4 against 16.9 / 11.2; SU(2) FP32 16^3 x 8
 // overrelaxation 1.9 against 2.6 with SP = 6.  The early launch hides the
@@ -753,7 +753,7 @@ cudaError_t launch_phase_T(const Geom &G, void *links, int group, const PhaseArg
     // shape 0 otherwise: the compiler's registers, or the form held to five
     // blocks per SM (shape 1) where that is the faster: SU(3) FP32 (us a phase,
     // heatbath / overrelaxation: 20^4 19.2 / 10.2 -> 17.2 / 9.6, 24^4 31.4 / 16.5
-    // -> 29.8 / 15.9, 32^4 92.8 / 54.9 -> 88.4 / 51.2) and SU(2) up to 100 000
+    // -> 29.9 / 16.5, 32^4 93.7 / 58.9 -> 89.1 / 57.1) and SU(2) up to 100 000
     // links (FP32 16^4 5.6 / 3.1 -> 5.1 / 2.4, FP64 6.9 / 4.0 -> 5.7 / 3.4; at 32^4
     // the FP64 heatbath 39.6 against 44.4); SU(3) FP64 spills (16^4 14.4 / 8.4
     // against 17.8 / 11.0)

@@ -29,7 +29,7 @@ def main():
                     help="after the rest, print qg_profile_kernels' per-launch times (this many launches per class)")
     ap.add_argument("--measure", default="",
                     help="comma list run after the phases: wilson_all (8x8, FP32 products), "
-                         "wilson_all64 (FP64 products), fmunu, action_profile, polyakov_profile, plaquette")
+                         "wilson_all64 (FP64 products), wilson (7x2), fmunu, action_profile, polyakov_profile, plaquette")
     a = ap.parse_args()
     cfg = Q.default_config(group=a.group, size=a.size, precision=a.precision, start=Q.START_COLD,
                            prng=Q.PRNG_PHILOX if a.prng == "philox" else Q.PRNG_RANLUX, beta=6.0, n_or=0,
@@ -50,6 +50,8 @@ def main():
             L.wilson_all(8, 8, fp64_products=False)
         elif m == "wilson_all64":
             L.wilson_all(8, 8, fp64_products=True)
+        elif m == "wilson":
+            L.wilson_sum(7, 2)
         elif m == "fmunu":
             L.fmunu(Q.FMUNU_H)
         elif m == "action_profile":
