@@ -111,16 +111,17 @@ def test_every_shape_in_the_graph_equals_single_phases(group, precision, size, m
 
 @pytest.mark.parametrize("group,precision", [(3, 0), (3, 1), (2, 0), (2, 1)])
 def test_the_tuner_times_small_lattices_as_the_sweep_runs_them(group, precision):
-    """at 8^4 a phase takes less than a launch by the host, in either form; in the graph the split one takes 0.5 to
-    0.7 of the other's time (its least ratio there: SU(3) FP32 heatbath, 6.8 to 9.4 us), and the tuner keeps it"""
+    """at 8^4 a phase takes less than a launch by the host, in either form.  In the graph the split heatbath takes
+    0.49 (SU(3) FP64) to 0.75 (SU(3) FP32: 6.9 to 9.2 us) of the other's time, 0.77 with the graph's start (some
+    4 us over 8 phases) in both; 0.85 leaves a tenth for the spread of the least of three.  (The overrelaxations lie
+    closer, 2.1 to 2.3 us for SU(2) FP32, so their order is left open.)"""
     kw = dict(group=group, precision=precision, size=(8, 8, 8, 8), beta=5.9 if group == 3 else 2.3, n_or=2,
               prng=Q.PRNG_PHILOX)
     L = Q.Lattice(Q.default_config(start=Q.START_HOT, randseries=7, reunit_every=2, **kw))
     L.seed()
     L.init(Q.START_HOT)
     t = L.tune()
-    assert t[0][0] < 0.9 * t[1][0] and t[0][1] < 0.9 * t[1][1], t
-    assert L.shapes() == (0, 0), t
+    assert t[0][0] < 0.85 * t[1][0] and L.shapes()[0] == 0, t
     L.sweep(3)
     assert np.array_equal(L.download(), chain(1, 3, **kw))
     L.close()
