@@ -420,7 +420,10 @@ __global__ void __launch_bounds__(kPhaseBlock, 1) k_phase_or_pair(Field<float> U
 // the rare later quads).  Operations and their order per value are those of
 // phase_site.  In a sweep's graph the launches are programmatic dependents:
 // a phase's indices and random numbers are computed under the end of the
-// phase before it.
+// phase before it.  A phase lets the next one start before it waits itself, so
+// a third may be resident while the first still writes; each waits for the end
+// of the one before, which ends after its own wait, and reads links after that
+// with ordinary loads only.
 constexpr int kSplitQuads = 6;
 
 // the functions of one quad that a Kennedy-Pendleton step uses, as a try
